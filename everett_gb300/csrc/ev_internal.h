@@ -141,13 +141,23 @@ struct PlanBlob {
   }
 };
 
+// Which qubits a tile holds (ev_tile.cu).
+struct TilePlan {
+  int k, L;
+  int nH;
+  uint8_t H[40];     // local positions L..k-1 map to global qubits H[0..nH)
+  int ncomp;
+  uint8_t comp[64];  // global qubits outside T, ascending
+};
+
 // One shared-memory tile pass or one fused-unitary pass of a planned run.
 struct SegStep {
   int fused = 0;        // 0: tile pass, 1: fused unitary
-  size_t off0 = 0;      // tile: TilePlan offset; fused: FusedDesc offset (in the blob)
+  TilePlan tile{};      // tile: its qubits
+  size_t off0 = 0;      // fused: FusedDesc offset (in the blob)
   size_t off1 = 0;      // tile: first op record; fused: matrix operands
   int nops = 0;         // tile: op records
-  int k = 0, L = 0;     // tile: tile bits, contiguous low bits; fused: k = qubits
+  int k = 0;            // fused: qubits per unitary
   int variant = 0;      // fused: EV_FUSED_*
   int tma = 0;          // fused: TMA-staged pipeline
   uint64_t count = 0;   // tile: tiles; fused: 128-row steps

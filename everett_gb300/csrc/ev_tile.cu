@@ -85,13 +85,14 @@ constexpr uint32_t kTileWaitLimit = 1u << 24;  // try_wait polls before giving u
 // EV_ERR_TIMEOUT) and ends the block after a bounded drain.
 template <typename V, bool BULK, int NT, int MINB>
 __global__ void __launch_bounds__(NT, MINB)
-    k_tile(V* __restrict__ s, uint64_t ntiles, const TilePlan* __restrict__ gplan,
-           const TileOp* __restrict__ gops, int nops, const uint8_t* pred, int* err) {
-  constexpr bool kStageOps = MINB < 3;
-  if (pred != nullptr && *pred == 0) return;
+    k_tile(V* __restrict__ s, uint64_t ntiles, const __grid_constant__ TilePlan plan,
+           const TileOp* __restrict__ gops, int nops, int* err) {
+  constexpr bool kStageOps = !(NT == 256 && MINB == 3);
+  // the next pass may start its own staging now; it waits below for this one
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ __align__(8) uint64_t bar;
-  const int k = gplan->k, L = gplan->L, nH = gplan->nH, ncomp = gplan->ncomp;
+  const int k = plan.k, L = plan.L, nH = plan.nH, ncomp = plan.ncomp;
   const uint32_t size = 1u << k;
   const uint32_t nrows = 1u << (k - L);
   const uint32_t rowbytes = uint32_t(sizeof(V)) << L;
@@ -116,17 +117,19 @@ __global__ void __launch_bounds__(NT, MINB)
       const int words = nops * int(sizeof(TileOp) / sizeof(uint4));
       for (int w = threadIdx.x; w < words; w += blockDim.x) dst[w] = src[w];
     }
-    if (threadIdx.x < 64) comp[threadIdx.x] = gplan->comp[threadIdx.x];
+    for (int w = threadIdx.x; w < 64; w += blockDim.x) comp[w] = plan.comp[w];
   }
   for (uint32_t h = threadIdx.x; h < nrows; h += blockDim.x) {
     uint64_t o = 0;
     for (int b = 0; b < nH; ++b)
-      if ((h >> b) & 1) o |= uint64_t(1) << gplan->H[b];
+      if ((h >> b) & 1) o |= uint64_t(1) << plan.H[b];
     offs[h] = o;
   }
   const uint32_t lowmask = (1u << L) - 1;
   uint32_t phase = 0;
   __syncthreads();
+  // the previous kernel of the stream has finished and its stores are visible
+  asm volatile("griddepcontrol.wait;" ::: "memory");
   for (uint64_t t = blockIdx.x; t < ntiles; t += gridDim.x) {
     uint64_t base = 0;
     for (int b = 0; b < ncomp; ++b)
@@ -163,6 +166,8 @@ __global__ void __launch_bounds__(NT, MINB)
           tile_quad_chain(tile, size, ops + o, run, nullptr);
         else if (run > 1 && op.ctype == CH_DIAG)
           tile_diag_chain(tile, size, ops + o, run, nullptr);
+        else if (run > 1 && NT < kTileThreads && kStageOps)
+          tile_chain_one(tile, size >> op.nins, ops + o, run, nullptr);
         else if (run > 1)
           tile_chain(tile, size >> op.nins, ops + o, run, nullptr);
         else
@@ -191,52 +196,96 @@ __global__ void __launch_bounds__(NT, MINB)
 }
 
 template <typename V, bool BULK, int NT, int MINB>
-static int launch_tile_as(ev_state* s, uint64_t ntiles, size_t smem, const TilePlan* dplan,
-                          const TileOp* dops, int nops, const uint8_t* pred) {
+static int launch_tile_as(ev_state* s, uint64_t ntiles, size_t smem, const TilePlan& plan,
+                          const TileOp* dops, int nops) {
   EV_TRY(prepare_smem_kernel(reinterpret_cast<const void*>(k_tile<V, BULK, NT, MINB>)));
-  int per_sm = 0;
-  EV_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_tile<V, BULK, NT, MINB>, NT,
-                                                        smem));
-  if (per_sm < 1) per_sm = 1;
-  uint64_t grid = uint64_t(s->num_sms) * per_sm;
-  if (grid > ntiles) grid = ntiles;
+  uint64_t grid = ntiles;
+  if (ntiles > uint64_t(s->num_sms)) {
+    int per_sm = 0;
+    EV_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_tile<V, BULK, NT, MINB>, NT,
+                                                          smem));
+    if (per_sm < 1) per_sm = 1;
+    grid = std::min(ntiles, uint64_t(s->num_sms) * per_sm);
+  }
   ProfScope prof(s, P_TILE, 2.0 * double(s->len()) * double(sizeof(V)));
   s->launches += 1;
   int* derr = reinterpret_cast<int*>(s->scratch.counter + 1);
-  k_tile<V, BULK, NT, MINB><<<unsigned(grid), NT, smem, s->stream>>>(
-      static_cast<V*>(s->amps), ntiles, dplan, dops, nops, pred, derr);
-  EV_CUDA(cudaGetLastError());
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(unsigned(grid));
+  cfg.blockDim = dim3(NT);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s->stream;
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &attr;
+  // Early launch only where the next pass's blocks find SMs of their own:
+  // with more blocks than that they land beside running ones, unevenly, and
+  // a pass lasts as long as its fullest SM (complex128, ms per depth-20
+  // circuit, early launch on / off: 14 qubits, 64 blocks, 0.61 / 0.64; 15
+  // qubits, 128 blocks, 0.85 / 0.68; 20 qubits, 304 blocks of 256 threads,
+  // 8.50 / 7.20).
+  cfg.numAttrs = 2 * grid <= uint64_t(s->num_sms) ? 1 : 0;
+  EV_CUDA(cudaLaunchKernelEx(&cfg, k_tile<V, BULK, NT, MINB>, static_cast<V*>(s->amps), ntiles,
+                             plan, dops, nops, derr));
   return EV_OK;
 }
 
+// Threads of a block: one per pair of a tile of up to 2^8 amplitudes, one per
+// quad above.
+static int tile_block(int k) { return k <= 9 ? 128 : k <= 11 ? 256 : kTileThreads; }
+
 template <typename V>
-static int launch_tile(ev_state* s, uint64_t ntiles, const TilePlan& plan, const TilePlan* dplan,
-                       const TileOp* dops, int nops, const uint8_t* pred) {
+static int launch_tile(ev_state* s, uint64_t ntiles, const TilePlan& plan, const TileOp* dops,
+                       int nops) {
   const size_t ops_at = (sizeof(V) * (size_t(1) << plan.k) +
                          sizeof(uint64_t) * (size_t(1) << (plan.k - plan.L)) + 15) & ~size_t(15);
   const bool bulk = tile_bulk_enabled();
   const int shape = tile_shape();
   if (shape == 1 && !bulk)
-    return launch_tile_as<V, false, 256, 3>(s, ntiles, ops_at + 64, dplan, dops, nops, pred);
+    return launch_tile_as<V, false, 256, 3>(s, ntiles, ops_at + 64, plan, dops, nops);
   const size_t smem = ops_at + sizeof(TileOp) * size_t(nops) + 64;
   if (shape == 2 && !bulk)
-    return launch_tile_as<V, false, kTileThreads, 1>(s, ntiles, smem, dplan, dops, nops, pred);
-  if (bulk) return launch_tile_as<V, true, kTileThreads, 2>(s, ntiles, smem, dplan, dops, nops, pred);
-  return launch_tile_as<V, false, kTileThreads, 2>(s, ntiles, smem, dplan, dops, nops, pred);
+    return launch_tile_as<V, false, kTileThreads, 1>(s, ntiles, smem, plan, dops, nops);
+  if (bulk) return launch_tile_as<V, true, kTileThreads, 2>(s, ntiles, smem, plan, dops, nops);
+  const int threads = tile_block(plan.k);
+  if (threads == 128) return launch_tile_as<V, false, 128, 4>(s, ntiles, smem, plan, dops, nops);
+  if (threads == 256) return launch_tile_as<V, false, 256, 2>(s, ntiles, smem, plan, dops, nops);
+  return launch_tile_as<V, false, kTileThreads, 2>(s, ntiles, smem, plan, dops, nops);
 }
 
-int default_tile_bits(int dtype) { return dtype == EV_C128 ? 12 : 13; }
+// Tile bits when the caller names none.  A complex128 pass is bound by the
+// FP64 and integer pipes of the SMs that hold a tile, so a register below
+// 2^19 amplitudes is cut into enough tiles to reach them all, at the price of
+// more passes (a few microseconds each); from 2^19 on, tiles of 2^12 fill
+// the GPU and the fewest passes win.  Measured, complex128, ms per depth-20
+// random-layer circuit (depth 10 at 10 qubits), tiles of 2^8 / 2^10 / 2^12:
+// 10 qubits 0.21 / 0.41 / -; 14 qubits 0.61 / 1.09 / 2.94; 17 qubits
+// 1.10 / 1.82 / 3.60; 18 qubits 2.24 / 2.00 / 5.5; 19 qubits 4.2 / 4.1 /
+// 4.0; 20 qubits 8.4 / 8.5 / 7.4.  complex64 (2^8 / 2^10 / 2^12 / 2^13): 14
+// qubits 0.22 / 0.24 / 0.45 / 0.76; 17 qubits 0.33 / 0.38 / 0.56 / 0.95; 18
+// qubits 0.56 / 0.43 / 0.70 / 0.99; 20 qubits 1.6 / 1.2 / 0.92 / 1.54; 22
+// qubits, depth 10, 3.3 / 2.0 / 1.9 / 1.7.
+int default_tile_bits(int dtype, int n) {
+  if (n <= 17) return 8;
+  if (n <= 18) return 10;
+  if (dtype == EV_C128) return 12;
+  return n <= 19 ? 10 : n <= 20 ? 12 : 13;
+}
 
 // Plans a gate run into tile passes; plans and records go into the blob.
 int plan_tiled(ev_state* s, const ev_circuit* c, uint64_t first, uint64_t last, int tile_bits,
                PlanBlob* blob, std::vector<SegStep>* out) {
   const int n = int(s->n);
-  int k = tile_bits > 0 ? tile_bits : default_tile_bits(s->dtype);
+  int k = tile_bits > 0 ? tile_bits : default_tile_bits(s->dtype, n);
   const int kcap = s->dtype == EV_C128 ? 13 : 14;  // tile + records within 227 KiB
   if (k > kcap) k = kcap;
   if (k < 2) k = 2;
   if (k > n) k = n;
-  const int L = std::min(k, 4);
+  // low qubits that every tile holds: whole lines of 2^4 amplitudes from HBM;
+  // a state that stays in the L2 cache is read in rows of 2^2 (17 qubits,
+  // complex128: 61 passes instead of 44, 1.12 ms against 1.10)
+  const int L = std::min(k, n <= 21 ? 2 : 4);
   // one op may need 2 data qubits beyond the low ones
   if (k - L < 2 && k < n) k = std::min(n, L + 2);
   // complex64 may reorder commuting ops; complex128 keeps the reference's order
@@ -244,7 +293,10 @@ int plan_tiled(ev_state* s, const ev_circuit* c, uint64_t first, uint64_t last, 
       plan_passes(c, first, last, n, k, L, uint64_t(kMaxPassOps), s->dtype == EV_C64);
   const uint64_t ntiles = uint64_t(1) << (n - k);
   const SoftLevels soft = tile_soft_levels();
-  const ChainSet chains = chain_set("EV_TILE_CHAIN", ChainSet{true, true, true});
+  // a quad chain occupies a thread per four amplitudes: where that leaves
+  // threads idle, pair chains finish sooner (14 qubits 0.94 -> 0.61 ms)
+  const bool quads = (1 << k) / 4 >= tile_block(k);
+  const ChainSet chains = chain_set("EV_TILE_CHAIN", ChainSet{true, quads, true});
   std::vector<TileOp> ops;
   for (const Pass& p : passes) {
     TilePlan plan{};
@@ -271,11 +323,9 @@ int plan_tiled(ev_state* s, const ev_circuit* c, uint64_t first, uint64_t last, 
     mark_chains(ops.data(), ops.size(), chains);
     SegStep st;
     st.fused = 0;
-    st.off0 = blob->add(&plan, sizeof(plan));
+    st.tile = plan;
     st.off1 = blob->add(ops.data(), ops.size() * sizeof(TileOp));
     st.nops = int(ops.size());
-    st.k = k;
-    st.L = L;
     st.count = ntiles;
     out->push_back(st);
   }
@@ -283,13 +333,9 @@ int plan_tiled(ev_state* s, const ev_circuit* c, uint64_t first, uint64_t last, 
 }
 
 int launch_tile_step(ev_state* s, const SegStep& st, const unsigned char* dblob) {
-  TilePlan plan{};
-  plan.k = st.k;
-  plan.L = st.L;
-  const TilePlan* dplan = reinterpret_cast<const TilePlan*>(dblob + st.off0);
   const TileOp* dops = reinterpret_cast<const TileOp*>(dblob + st.off1);
-  if (s->dtype == EV_C128) return launch_tile<double2>(s, st.count, plan, dplan, dops, st.nops, nullptr);
-  return launch_tile<float2>(s, st.count, plan, dplan, dops, st.nops, nullptr);
+  if (s->dtype == EV_C128) return launch_tile<double2>(s, st.count, st.tile, dops, st.nops);
+  return launch_tile<float2>(s, st.count, st.tile, dops, st.nops);
 }
 
 // ---- device check of the integer-pipe product ------------------------------------

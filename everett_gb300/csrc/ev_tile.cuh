@@ -76,14 +76,6 @@ __host__ __device__ __forceinline__ const double* rec_m(const TileOp& op, const 
 }
 __host__ __device__ __forceinline__ uint32_t rec_sok(const TileOp& op) { return op.sok; }
 
-struct TilePlan {
-  int k, L;
-  int nH;
-  uint8_t H[40];     // local positions L..k-1 map to global qubits H[0..nH)
-  int ncomp;
-  uint8_t comp[64];  // global qubits outside T, ascending
-};
-
 // Entry i of a record's matrix.  complex128 records hold f64 [re, im]
 // pairs; complex64 records hold f32 pairs, rounded once on the host
 // (pack_f32_matrix) because GB300 runs f64 -> f32 conversions at its FP64
@@ -308,7 +300,7 @@ __device__ __forceinline__ void pair_fp(const double* mm, V& a0, V& a1) {
 // plain arithmetic.  The two pairs are updated one after the other: a
 // straight-line block over both needs more registers than a 64-register
 // thread has, and its spills cost more than its extra overlap gains.
-template <int K1, typename V, typename Op>
+template <int K1, int PAIRS, typename V, typename Op>
 __device__ __forceinline__ void chain_rec(const Op& op, const double* mats, V& a0, V& a1, V& b0,
                                           V& b1) {
   const double* mm = rec_m(op, mats);
@@ -328,17 +320,42 @@ __device__ __forceinline__ void chain_rec(const Op& op, const double* mats, V& a
       const bool both = op.soft >= 2;
       const int nadd = op.soft > 2 ? op.soft - 2 : 0;
       soft_pair<K1>(a0, a1, f, both, nadd);
-      soft_pair<K1>(b0, b1, f, both, nadd);
+      if constexpr (PAIRS == 2) soft_pair<K1>(b0, b1, f, both, nadd);
       return;
     }
   }
   pair_fp<K1>(mm, a0, a1);
-  pair_fp<K1>(mm, b0, b1);
+  if constexpr (PAIRS == 2) pair_fp<K1>(mm, b0, b1);
 }
 
 template <typename V, typename Op>
 __device__ __forceinline__ void chain_rec_any(const Op& op, const double* mats, V& a0, V& a1,
                                               V& b0, V& b1);
+
+// chain_rec_any on one pair.
+template <typename V, typename Op>
+__device__ __forceinline__ void chain_rec_one(const Op& op, const double* mats, V& a0, V& a1);
+
+// tile_chain for blocks with a thread for (nearly) every pair of the tile: a
+// thread holds one pair at a time, so no lane repeats another's work and the
+// chain's latency is that of one pair.
+template <typename V, typename Op>
+__device__ void tile_chain_one(V* t, uint32_t count, const Op* ops, int run, const double* mats) {
+  const Op& op0 = ops[0];
+  const uint32_t tbit = 1u << op0.p0, lmask = op0.lmask;
+  const int nins = op0.nins;
+  const uint64_t ins = op0.ins;
+  const int ins_first = int(ins & 15);
+  for (uint32_t i = threadIdx.x; i < count; i += blockDim.x) {
+    uint32_t j = ins0(i, ins_first);
+    for (int q = 1; q < nins; ++q) j = ins0(j, int((ins >> (4 * q)) & 15));
+    j |= lmask;
+    V a0 = t[j], a1 = t[j | tbit];
+    for (int r = 0; r < run; ++r) chain_rec_one(ops[r], mats, a0, a1);
+    t[j] = a0;
+    t[j | tbit] = a1;
+  }
+}
 
 // A chain of `run` 1-qubit records that share their target and controls:
 // each thread loads two pairs, applies every record of the chain to them in
@@ -374,18 +391,27 @@ __device__ void tile_chain(V* t, uint32_t count, const Op* ops, int run, const d
   }
 }
 
-// chain_rec for the record's kind.
+// chain_rec for the record's kind, on one pair or two.
+template <int PAIRS, typename V, typename Op>
+__device__ __forceinline__ void chain_rec_kind(const Op& op, const double* mats, V& a0, V& a1,
+                                               V& b0, V& b1) {
+  switch (op.k1) {
+    case K1_DENSE: chain_rec<K1_DENSE, PAIRS>(op, mats, a0, a1, b0, b1); break;
+    case K1_REAL: chain_rec<K1_REAL, PAIRS>(op, mats, a0, a1, b0, b1); break;
+    case K1_DIAG: chain_rec<K1_DIAG, PAIRS>(op, mats, a0, a1, b0, b1); break;
+    case K1_PHASE: chain_rec<K1_PHASE, PAIRS>(op, mats, a0, a1, b0, b1); break;
+    case K1_ANTI: chain_rec<K1_ANTI, PAIRS>(op, mats, a0, a1, b0, b1); break;
+    default: break;  // identity
+  }
+}
 template <typename V, typename Op>
 __device__ __forceinline__ void chain_rec_any(const Op& op, const double* mats, V& a0, V& a1,
                                               V& b0, V& b1) {
-  switch (op.k1) {
-    case K1_DENSE: chain_rec<K1_DENSE>(op, mats, a0, a1, b0, b1); break;
-    case K1_REAL: chain_rec<K1_REAL>(op, mats, a0, a1, b0, b1); break;
-    case K1_DIAG: chain_rec<K1_DIAG>(op, mats, a0, a1, b0, b1); break;
-    case K1_PHASE: chain_rec<K1_PHASE>(op, mats, a0, a1, b0, b1); break;
-    case K1_ANTI: chain_rec<K1_ANTI>(op, mats, a0, a1, b0, b1); break;
-    default: break;  // identity
-  }
+  chain_rec_kind<2>(op, mats, a0, a1, b0, b1);
+}
+template <typename V, typename Op>
+__device__ __forceinline__ void chain_rec_one(const Op& op, const double* mats, V& a0, V& a1) {
+  chain_rec_kind<1>(op, mats, a0, a1, a0, a1);
 }
 
 // A chain of `run` uncontrolled 1-qubit records whose targets are two local
@@ -546,8 +572,6 @@ inline uint64_t data_qubits(const ev_op& op) {
 
 inline int popc(uint64_t x) { return __builtin_popcountll(x); }
 
-// Greedy: extend the current pass while the union of data qubits (plus the
-// L lowest qubits) fits in k, then fill T with the lowest unused qubits.
 // Every qubit an op reads or writes (data qubits and controls).
 inline uint64_t all_qubits(const ev_circuit* c, const ev_op& op) {
   uint64_t m = data_qubits(op);
@@ -556,49 +580,64 @@ inline uint64_t all_qubits(const ev_circuit* c, const ev_op& op) {
   return m;
 }
 
-// Greedy pass planning over ops [first, last).  In order (reorder = false)
-// a pass is the longest run of consecutive ops whose data qubits, with the
-// L lowest qubits, fit in k; this keeps every amplitude's sequence of
-// roundings, so complex128 results stay bit-identical.  With reorder = true
-// a pass also takes later ops that touch no qubit of an op left behind
-// (they commute with everything they jump), which packs many more gates per
-// pass at the cost of a different rounding order.  T is filled up to k with
-// the lowest unused qubits.
+// A record that only moves amplitudes or flips their signs (CNOT, CZ, SWAP):
+// it commutes bit for bit with every record that shares no qubit with it,
+// since each amplitude of the other record's pairs is moved (and signed)
+// along with its partner.
+inline bool moves_only(const ev_op& op) {
+  if (op.kind != EV_OP_APPLY2) return false;
+  const Kind2 k = classify2(op.m);
+  return k == K2_CNOT || k == K2_CZ || k == K2_SWAP;
+}
+
+// Greedy pass planning over ops [first, last): a pass takes, in circuit
+// order, every pending op that fits (its data qubits with the L lowest and
+// those already chosen are at most k) and touches no qubit of an op left
+// behind.  reorder = true lets any such op jump (they commute in exact
+// arithmetic; the rounding order changes).  Otherwise an op jumps only when
+// the jump changes no bit: it moves amplitudes only, or so do all the ops
+// left behind; arithmetic records keep their order among themselves.  On
+// random layers with CNOT bricks that halves the passes against taking only
+// the next consecutive ops (17 qubits, depth 20, k = 8: 130 -> 65; 26
+// qubits, depth 10, k = 12: 55 -> 31), because a brick no longer ends the
+// run of rotations around it.  T is filled up to k with the lowest unused
+// qubits.
 inline std::vector<Pass> plan_passes(const ev_circuit* c, uint64_t first, uint64_t last, int n,
                                      int k, int L, uint64_t max_ops = 48, bool reorder = false) {
   std::vector<Pass> passes;
   const uint64_t low = (L >= 64) ? ~0ull : ((uint64_t(1) << L) - 1);
   const uint64_t everything = n >= 64 ? ~0ull : ((uint64_t(1) << n) - 1);
-  std::vector<uint64_t> pending;
-  for (uint64_t j = first; j < last; ++j) pending.push_back(j);
-  size_t head = 0;  // in-order mode consumes pending from the front
-  while (head < pending.size()) {
+  struct Pending {
+    uint64_t op, all, data;
+    bool moves;
+  };
+  std::vector<Pending> pending, rest;
+  pending.reserve(last - first);
+  for (uint64_t j = first; j < last; ++j) {
+    const ev_op& op = c->ops[j];
+    pending.push_back({j, all_qubits(c, op), data_qubits(op), reorder || moves_only(op)});
+  }
+  while (!pending.empty()) {
     Pass p;
     uint64_t set = low, blocked = 0;
-    if (!reorder) {
-      while (head < pending.size() && p.ops.size() < max_ops) {
-        const uint64_t want = set | data_qubits(c->ops[pending[head]]);
-        if (popc(want) > k) break;
-        set = want;
-        p.ops.push_back(pending[head++]);
+    bool behind = false;  // an arithmetic op has been left behind
+    rest.clear();
+    for (size_t i = 0; i < pending.size(); ++i) {
+      const Pending& e = pending[i];
+      if (blocked == everything || p.ops.size() >= max_ops) {  // nothing more can join
+        rest.insert(rest.end(), pending.begin() + ptrdiff_t(i), pending.end());
+        break;
       }
-    } else {
-      std::vector<uint64_t> rest;
-      for (size_t i = head; i < pending.size(); ++i) {
-        const ev_op& op = c->ops[pending[i]];
-        const uint64_t aq = all_qubits(c, op), dq = data_qubits(op);
-        if ((aq & blocked) == 0 && popc(set | dq) <= k && p.ops.size() < max_ops &&
-            blocked != everything) {
-          set |= dq;
-          p.ops.push_back(pending[i]);
-        } else {
-          blocked |= aq;
-          rest.push_back(pending[i]);
-        }
+      if ((e.all & blocked) == 0 && (e.moves || !behind) && popc(set | e.data) <= k) {
+        set |= e.data;
+        p.ops.push_back(e.op);
+      } else {
+        blocked |= e.all;
+        behind = behind || !e.moves;
+        rest.push_back(e);
       }
-      pending.swap(rest);
-      head = 0;
     }
+    pending.swap(rest);
     for (int q = 0; q < n && popc(set) < k; ++q) set |= uint64_t(1) << q;
     p.tset = set;
     passes.push_back(std::move(p));

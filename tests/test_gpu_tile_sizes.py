@@ -1,0 +1,65 @@
+"""The tile pass's default tile per register size (tiles of 2^8, 2^10 and 2^12
+amplitudes, rows of 2^2 or 2^4) against the oracle, on both sides of every
+edge of the rule, with moves (CNOT, CZ, SWAP) between arithmetic gates on
+other qubits, which the pass planner carries across each other.
+
+complex128 equals the oracle (==: the carried moves change no bit);
+complex64 keeps fidelity >= 1 - 1e-6."""
+import numpy as np
+import pytest
+
+import oracle as O
+from everett_gb300 import Circuit, CudaStateVectorBackend, Gate1, Gate2, algorithms
+
+pytestmark = pytest.mark.gpu
+
+
+def interleaved(n, seed, count):
+    rng = np.random.default_rng(seed)
+    c = Circuit(n)
+    for q in range(n):
+        c.h(q)
+    for _ in range(count):
+        q = [int(v) for v in rng.choice(n, min(n, 4), replace=False)]
+        k = int(rng.integers(0, 8))
+        if n < 2 or k < 2:
+            c.rz(q[0], rng.uniform(0, 6)).ry(q[0], rng.uniform(0, 6))
+        elif k < 5:
+            c.gate2([Gate2.cnot(), Gate2.cz(), Gate2.swap()][k - 2], q[0], q[1])
+        elif k == 5:
+            c.controlled(q[1:3], Gate1.ry(0.3), q[0])
+        elif k == 6:
+            c.gate2(Gate2.rzz(rng.uniform(0, 6)), q[0], q[1])
+        else:
+            c.gate2(Gate2.controlled(Gate1.rx(0.9)), q[0], q[1])
+    return c
+
+
+@pytest.mark.parametrize("n", [1, 2, 3, 7, 8, 9, 10, 16, 17, 18, 19, 21, 22])
+def test_default_tiles_bit_exact(gpu, n):
+    c = interleaved(n, n, 160 if n < 18 else 60)
+    want, _, rc = O.run_seeded(c, 0, parallel=True)
+    assert rc == 0
+    got = CudaStateVectorBackend.run(c).state().amplitudes()
+    assert np.array_equal(got, want)
+    single = CudaStateVectorBackend.run(c, dtype="complex64").state().amplitudes()
+    fid = abs(np.vdot(want, single)) ** 2 / (np.vdot(single, single).real * np.vdot(want, want).real)
+    assert fid > 1 - 1e-6
+
+
+@pytest.mark.parametrize("dtype", ["complex128", "complex64"])
+def test_default_tiles_replayed(gpu, dtype):
+    """A prepared run with measurements between its tile passes (passes that
+    may start before the previous kernel ends, captured into a graph) equals
+    the same run launched kernel by kernel."""
+    n = 11
+    c = Circuit.with_classical(n, 2)
+    c.compose(interleaved(n, 5, 40)).measure(3, 0).x_if(0, 7)
+    c.compose(algorithms.qft(n)).measure(n - 1, 1)
+    st = CudaStateVectorBackend.run_seeded(c, 9, dtype=dtype)
+    again = CudaStateVectorBackend(n, dtype=dtype).state()
+    prepared = CudaStateVectorBackend.prepare(again, c)
+    for _ in range(3):
+        assert prepared.launch(9) == st.classical()
+        assert np.array_equal(again.amplitudes(), st.state().amplitudes())
+    prepared.close()
