@@ -41,12 +41,14 @@ bool debug_enabled();
 // Upper bound on blocks of a reduction grid (partials live in the state's
 // scratch area).
 constexpr int kMaxRedBlocks = 2048;
+// Reduction results that can wait on the device before the host reads them.
+constexpr int kMaxResults = 1024;
 
 // Per-state device scratch: reduction partials, measurement results and the
 // device-resident classical register of a run.
 struct Scratch {
   double* partials;   // kMaxRedBlocks * 4 doubles
-  double* result;     // 8 doubles: reduction results
+  double* result;     // kMaxResults doubles: reduction results
   double* meas;       // 4 doubles: p1, scale, outcome (as double), u
   uint8_t* pred;      // 64 bytes: combined predicates of nested IfClassic
   uint32_t* counter;  // 4 words: uniforms consumed by device-side measurement

@@ -112,3 +112,32 @@ def test_marginal_low_and_phase_estimation(gpu, dtype):
         for b1 in (False, True):
             ex = CudaStateVectorBackend.run(algorithms.superdense_circuit(b0, b1))
             assert list(ex.classical()) == [b0, b1]
+
+
+@pytest.mark.parametrize("dtype", ["complex128", "complex64"])
+@pytest.mark.parametrize("n", [1, 2, 4, 5, 8, 9, 11, 12, 13, 19])
+def test_many_groups_from_one_read(gpu, n, dtype):
+    """Terms of many X parts evaluated from shared-memory tiles (each within
+    the tile's qubits), beside X parts too wide for a tile and more Z-only
+    terms than one pass takes: registers below, at and above a tile's 2^11
+    (complex128) and 2^12 (complex64) amplitudes, both Y parities, signs."""
+    rng = np.random.default_rng(n)
+    amps, _, _ = O.run_seeded(workloads.random_layers(n, 3, seed=n + 5), parallel=True)
+    st = State.from_amplitudes(amps, dtype=dtype)
+    ref = np.ascontiguousarray(st.amplitudes())
+    texts = []
+    for q in range(n):  # every site, and strings from it to the far end
+        for p in "XY":
+            texts.append("I" * q + p + "I" * (n - q - 1))
+        texts.append("-" + "I" * q + "Y" + "Z" * (n - q - 1))
+    for q in range(n - 1):
+        texts += ["I" * q + p + "I" * (n - q - 2) for p in ("ZZ", "XX", "XY", "YY", "ZX")]
+    ps = [PauliString.parse(t) for t in texts] + random_paulis(rng, n, 6)
+    ps += [PauliString([False] * n, rng.integers(0, 2, n).astype(bool), bool(rng.integers(0, 2)))
+           for _ in range(25)]
+    ps = [ps[i] for i in rng.permutation(len(ps))]
+    got = st.pauli_expectation(ps)
+    for p, g in zip(ps, got):
+        xm, zm = p.masks()
+        want = O.pauli_expectation(ref, xm, zm, p.neg)
+        assert abs(g - want) < 1e-12, (n, dtype, str(p), g, want)
