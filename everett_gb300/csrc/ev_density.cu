@@ -171,14 +171,108 @@ __device__ __forceinline__ void right2_any(const double2* u, const SoftU1& f, do
   }
 }
 
-// rho -> U rho U^dagger on qubit t; with mask != 0 the left product applies
-// to rows whose bits in mask are all set, the right product to such columns.
-__global__ void __launch_bounds__(kDmThreads)
-    k_dm_1q(double2* __restrict__ rho, int n, int t, U1 u, uint64_t mask, const uint8_t* pred) {
+// A channel whose Kraus operators are all real multiples of I, X, Y or Z, in
+// one or two magnitudes (depolarizing, bit flip, dephasing).  With K = c P
+// the left and right products each multiply every part of the block once by
+// c (up to exact signs, swaps and the two factors of i of a Y, which meet),
+// so K rho K^dagger is +-t_c of the element or of the one opposite, with
+// t_c(x) = RN(c RN(c x)): the three error terms of a depolarizing channel
+// share one t_c per element.  8 products per element instead of 16 for that
+// channel, and the same sums in the same order.
+struct PauliChannel {
+  double scale[2];
+  int n;                 // operators; 0: no channel
+  uint8_t second[EV_MAX_KRAUS], swap[EV_MAX_KRAUS], neg[EV_MAX_KRAUS];
+};
+
+__device__ __forceinline__ bool is_zero(double2 x) {  // tested as bits, off the FP64 pipe
+  return ((softfp::to_bits(x.x) | softfp::to_bits(x.y)) << 1) == 0;
+}
+// RN(c RN(c x)); a zero stays itself, an operand outside the integer-pipe
+// domain takes the FP64 pipe
+__device__ __forceinline__ double twice(double c, const softfp::Unpacked& cu, double x) {
+  const softfp::Unpacked ux = softfp::unpack(x);
+  if (cu.ok & ux.ok) {
+    const double m = softfp::mul(cu, ux);
+    const softfp::Unpacked um = softfp::unpack(m);
+    return um.ok ? softfp::mul(cu, um) : __dmul_rn(c, m);
+  }
+  // tested as bits: comparisons of doubles run on the FP64 pipe
+  return (softfp::to_bits(x) << 1) == 0 ? x : __dmul_rn(c, __dmul_rn(c, x));
+}
+__device__ __forceinline__ bool not_finite(double2 x) {
+  const uint32_t inf = 0x7FF00000u;
+  return (uint32_t(softfp::to_bits(x.x) >> 32) & inf) == inf ||
+         (uint32_t(softfp::to_bits(x.y) >> 32) & inf) == inf;
+}
+
+// The channel on the block e = (00, 01, 10, 11).  A NaN or an infinity takes
+// the products of the general form (the FMA form lets it reach both parts).
+__device__ __forceinline__ void pauli_channel(const PauliChannel& ch, double2 (&e)[4]) {
+  if (not_finite(e[0]) | not_finite(e[1]) | not_finite(e[2]) | not_finite(e[3])) {
+    double2 sum[4];
+    for (int k = 0; k < ch.n; ++k) {
+      const double c = ch.scale[ch.second[k]];
+      const double2 d0 = make_double2(ch.swap[k] ? 0.0 : c, 0.0);
+      const double2 d3 = make_double2(ch.swap[k] ? 0.0 : ch.neg[k] ? -c : c, 0.0);
+      const double2 o1 = ch.swap[k] ? (ch.neg[k] ? make_double2(0.0, -c) : make_double2(c, 0.0))
+                                    : make_double2(0.0, 0.0);
+      const double2 o2 = ch.swap[k] && ch.neg[k] ? make_double2(0.0, c) : o1;
+      const double2 u[4] = {d0, o1, o2, d3};
+      double2 x[4] = {e[0], e[1], e[2], e[3]};
+      left2(u, x[0], x[2]);
+      left2(u, x[1], x[3]);
+      right2(u, x[0], x[1]);
+      right2(u, x[2], x[3]);
+      for (int q = 0; q < 4; ++q) sum[q] = k == 0 ? x[q] : cadd(sum[q], x[q]);
+    }
+    for (int q = 0; q < 4; ++q) e[q] = sum[q];
+    return;
+  }
+  const softfp::Unpacked c0 = softfp::unpack(ch.scale[0]), c1 = softfp::unpack(ch.scale[1]);
+  const bool two = softfp::to_bits(ch.scale[1]) != 0;  // uniform
+  double2 t0[4], t1[4];
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    t0[q] = make_double2(twice(ch.scale[0], c0, e[q].x), twice(ch.scale[0], c0, e[q].y));
+    t1[q] = two ? make_double2(twice(ch.scale[1], c1, e[q].x), twice(ch.scale[1], c1, e[q].y))
+                : t0[q];
+  }
+  for (int k = 0; k < ch.n; ++k) {  // uniform branches
+    const bool b = ch.second[k], x = ch.swap[k];
+    double2 v[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+      v[q] = x ? (b ? t1[3 - q] : t0[3 - q]) : (b ? t1[q] : t0[q]);
+    if (ch.neg[k]) {
+      v[1] = make_double2(-v[1].x, -v[1].y);
+      v[2] = make_double2(-v[2].x, -v[2].y);
+    }
+#pragma unroll
+    for (int q = 0; q < 4; ++q) e[q] = k == 0 ? v[q] : cadd(e[q], v[q]);
+  }
+}
+
+// rho -> U rho U^dagger on qubit t (GATE), then a Pauli channel on t
+// (ch.n > 0) while the block is in registers; with mask != 0 the left product
+// applies to rows whose bits in mask are all set, the right product to such
+// columns.  Bound: the FP64 pipe (6 adds per element of a depolarizing
+// channel; 55-60 % busy) beside the integer pipes' products.  Depolarizing
+// noise after every gate, 11 qubits (rho in the L2 cache), from |0..0>, mean
+// of a run's launches: gate 87 us and channel 281 us in two passes -> 135 us
+// in one; the channel alone (after 2-qubit gates) 281 -> 109 us.  Three
+// blocks per SM (80 registers, ~200 bytes of spills) against two: 121 -> 109
+// us.
+template <bool GATE>
+__global__ void __launch_bounds__(kDmThreads, 3)
+    k_dm_1q(double2* __restrict__ rho, int n, int t, U1 u, uint64_t mask,
+            const __grid_constant__ PauliChannel ch, const uint8_t* pred) {
   if (dm_skip(pred)) return;
   __shared__ SoftU1 su;
-  if (threadIdx.x == 0) soft_u1(u.m, &su);
-  __syncthreads();
+  if (GATE) {
+    if (threadIdx.x == 0) soft_u1(u.m, &su);
+    __syncthreads();
+  }
   const SoftU1& f = su;
   const uint64_t half = uint64_t(1) << (n - 1), blocks = half * half;
   const uint64_t dim = uint64_t(1) << n, bit = uint64_t(1) << t;
@@ -186,20 +280,25 @@ __global__ void __launch_bounds__(kDmThreads)
   for (uint64_t b = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; b < blocks; b += stride) {
     const uint64_t r0 = insert0(b >> (n - 1), t), c0 = insert0(b & (half - 1), t);
     const uint64_t r1 = r0 | bit, c1 = c0 | bit;
-    double2 e00 = rho[r0 * dim + c0], e01 = rho[r0 * dim + c1];
-    double2 e10 = rho[r1 * dim + c0], e11 = rho[r1 * dim + c1];
-    if ((r0 & mask) == mask) {
-      left2_any(u.m, f, e00, e10);
-      left2_any(u.m, f, e01, e11);
+    double2 e[4] = {rho[r0 * dim + c0], rho[r0 * dim + c1], rho[r1 * dim + c0], rho[r1 * dim + c1]};
+    // a block of zeros stays one (most of rho until every qubit has been
+    // rotated; a zero operand would take the FP64 pipe)
+    if (is_zero(e[0]) & is_zero(e[1]) & is_zero(e[2]) & is_zero(e[3])) continue;
+    if (GATE) {
+      if ((r0 & mask) == mask) {
+        left2_any(u.m, f, e[0], e[2]);
+        left2_any(u.m, f, e[1], e[3]);
+      }
+      if ((c0 & mask) == mask) {
+        right2_any(u.m, f, e[0], e[1]);
+        right2_any(u.m, f, e[2], e[3]);
+      }
     }
-    if ((c0 & mask) == mask) {
-      right2_any(u.m, f, e00, e01);
-      right2_any(u.m, f, e10, e11);
-    }
-    rho[r0 * dim + c0] = e00;
-    rho[r0 * dim + c1] = e01;
-    rho[r1 * dim + c0] = e10;
-    rho[r1 * dim + c1] = e11;
+    if (ch.n > 0) pauli_channel(ch, e);
+    rho[r0 * dim + c0] = e[0];
+    rho[r0 * dim + c1] = e[1];
+    rho[r1 * dim + c0] = e[2];
+    rho[r1 * dim + c1] = e[3];
   }
 }
 
@@ -551,13 +650,56 @@ int dm_reduce_diag(const ev_dm* d, int k, const uint8_t* pred) {
   return EV_OK;
 }
 
-int dm_unitary_1q(ev_dm* d, uint64_t t, const double m[8], uint64_t mask, const uint8_t* pred) {
+// The channel as a PauliChannel, if it is one: every operator a real multiple
+// of I, X, Z or an imaginary antisymmetric one (Y), in at most two magnitudes.
+bool as_pauli(const ev_channel& ch, PauliChannel* out) {
+  *out = PauliChannel{};
+  int scales = 0;
+  for (uint32_t k = 0; k < ch.nops; ++k) {
+    const double* m = ch.k[k];  // [re, im] of 00, 01, 10, 11
+    const bool diag = m[2] == 0 && m[3] == 0 && m[4] == 0 && m[5] == 0 && m[1] == 0 && m[7] == 0;
+    const bool anti = m[0] == 0 && m[1] == 0 && m[6] == 0 && m[7] == 0;
+    double c = 0.0;
+    bool neg = false;
+    if (diag && (m[6] == m[0] || m[6] == -m[0])) {
+      c = m[0];
+      neg = m[6] != m[0];
+    } else if (anti && m[3] == 0 && m[5] == 0 && m[2] == m[4]) {
+      c = m[2];
+    } else if (anti && m[2] == 0 && m[4] == 0 && m[3] == -m[5]) {
+      c = m[5];
+      neg = true;
+    } else {
+      return false;
+    }
+    c = std::fabs(c);
+    if (!(c > 0.0 && c <= 1.7976931348623157e308)) return false;
+    int at = 0;
+    while (at < scales && out->scale[at] != c) ++at;
+    if (at == scales) {
+      if (scales == 2) return false;
+      out->scale[scales++] = c;
+    }
+    out->second[k] = uint8_t(at);
+    out->swap[k] = anti;
+    out->neg[k] = neg;
+  }
+  out->n = int(ch.nops);
+  return ch.nops > 0;
+}
+
+// A gate on t and, while its blocks are in registers, the channel after it on
+// t if it is a Pauli channel; *applied tells whether that channel is done.
+int dm_unitary_1q(ev_dm* d, uint64_t t, const double m[8], uint64_t mask, const PauliChannel* ch,
+                  const uint8_t* pred, bool* applied) {
+  *applied = false;
   if (mask == 0 && classify1(m) == K1_IDENT) return EV_OK;  // U = I: exact no-op
   U1 u;
   for (int e = 0; e < 4; ++e) u.m[e] = make_double2(m[2 * e], m[2 * e + 1]);
   const uint64_t half = d->dim() / 2;
-  k_dm_1q<<<dm_grid(d, half * half), kDmThreads, 0, d->stream>>>(d->rho, int(d->n), int(t), u,
-                                                                   mask, pred);
+  *applied = ch != nullptr;
+  k_dm_1q<true><<<dm_grid(d, half * half), kDmThreads, 0, d->stream>>>(
+      d->rho, int(d->n), int(t), u, mask, ch ? *ch : PauliChannel{}, pred);
   EV_CUDA(cudaGetLastError());
   return EV_OK;
 }
@@ -579,13 +721,21 @@ int dm_unitary_2q(ev_dm* d, uint64_t a, uint64_t b, const double m[32], const ui
   return EV_OK;
 }
 
-int dm_channel(ev_dm* d, const ev_channel& ch, uint64_t t, const uint8_t* pred) {
+// pauli: the channel as a PauliChannel, or null
+int dm_channel(ev_dm* d, const ev_channel& ch, const PauliChannel* pauli, uint64_t t,
+               const uint8_t* pred) {
   if (ch.nops == 0) return EV_OK;
+  const uint64_t half = d->dim() / 2;
+  if (pauli != nullptr) {
+    k_dm_1q<false><<<dm_grid(d, half * half), kDmThreads, 0, d->stream>>>(
+        d->rho, int(d->n), int(t), U1{}, 0, *pauli, pred);
+    EV_CUDA(cudaGetLastError());
+    return EV_OK;
+  }
   KrausSet ks;
   ks.nops = int(ch.nops);
   for (uint32_t k = 0; k < ch.nops; ++k)
     for (int e = 0; e < 4; ++e) ks.k[k][e] = make_double2(ch.k[k][2 * e], ch.k[k][2 * e + 1]);
-  const uint64_t half = d->dim() / 2;
   k_dm_channel<<<dm_grid(d, half * half), kDmThreads, 0, d->stream>>>(d->rho, int(d->n), int(t),
                                                                        ks, pred);
   EV_CUDA(cudaGetLastError());
@@ -620,6 +770,10 @@ int dm_run_ops(ev_dm* d, const ev_circuit* c, const ev_noise_model* nz, uint64_t
   if (!nz) nz = &kIdeal;
   if (nz->after_1q.nops > EV_MAX_KRAUS || nz->after_2q.nops > EV_MAX_KRAUS)
     return fail(EV_ERR_INVALID_ARGUMENT, "at most %d Kraus operators per channel", EV_MAX_KRAUS);
+  PauliChannel pauli1, pauli2;
+  const PauliChannel* p1 = as_pauli(nz->after_1q, &pauli1) ? &pauli1 : nullptr;
+  const PauliChannel* p2 = as_pauli(nz->after_2q, &pauli2) ? &pauli2 : nullptr;
+  bool applied = false;
   DmBuffers rb;
   rb.stream = d->stream;
   uint64_t nmeas = 0, nif = 0;
@@ -663,21 +817,21 @@ int dm_run_ops(ev_dm* d, const ev_circuit* c, const ev_noise_model* nz, uint64_t
     const ev_op& op = c->ops[pos];
     switch (op.kind) {
       case EV_OP_APPLY1:  // density_matrix.rs:101-107
-        EV_TRY(dm_unitary_1q(d, op.q0, op.m, 0, pred));
-        EV_TRY(dm_channel(d, nz->after_1q, op.q0, pred));
+        EV_TRY(dm_unitary_1q(d, op.q0, op.m, 0, p1, pred, &applied));
+        if (!applied) EV_TRY(dm_channel(d, nz->after_1q, p1, op.q0, pred));
         break;
       case EV_OP_APPLY2:  // density_matrix.rs:109-117
         EV_TRY(dm_unitary_2q(d, op.q0, op.q1, op.m, pred));
-        EV_TRY(dm_channel(d, nz->after_2q, op.q0, pred));
-        EV_TRY(dm_channel(d, nz->after_2q, op.q1, pred));
+        EV_TRY(dm_channel(d, nz->after_2q, p2, op.q0, pred));
+        EV_TRY(dm_channel(d, nz->after_2q, p2, op.q1, pred));
         break;
       case EV_OP_CONTROLLED: {  // density_matrix.rs:119-132
         uint64_t mask = 0;
         for (uint32_t j = 0; j < op.nctrl; ++j) mask |= uint64_t(1) << c->ctrl_pool[op.ctrl_off + j];
-        EV_TRY(dm_unitary_1q(d, op.q0, op.m, mask, pred));
-        EV_TRY(dm_channel(d, nz->after_1q, op.q0, pred));
+        EV_TRY(dm_unitary_1q(d, op.q0, op.m, mask, p1, pred, &applied));
+        if (!applied) EV_TRY(dm_channel(d, nz->after_1q, p1, op.q0, pred));
         for (uint32_t j = 0; j < op.nctrl; ++j)
-          EV_TRY(dm_channel(d, nz->after_1q, c->ctrl_pool[op.ctrl_off + j], pred));
+          EV_TRY(dm_channel(d, nz->after_1q, p1, c->ctrl_pool[op.ctrl_off + j], pred));
         break;
       }
       case EV_OP_MEASURE:  // density_matrix.rs:134-158

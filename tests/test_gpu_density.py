@@ -97,6 +97,38 @@ def test_larger_registers_without_controls(gpu):
         assert np.array_equal(got, want), n
 
 
+_I, _X = np.eye(2), np.array([[0, 1], [1, 0]])
+_Y, _Z = np.array([[0, -1j], [1j, 0]]), np.diag([1, -1])
+PAULI_CHANNELS = {
+    "one operator": [0.9 * _Y],
+    "one magnitude": [0.5 * _Z, -0.5 * _I, 0.5 * _X, -0.5 * _Y],
+    "two magnitudes": [0.1 * _X, 0.9 * _I, -0.1 * _Z, 0.1 * _Y, 0.9 * _Z],
+    "three magnitudes": [0.8 * _I, 0.2 * _X, 0.3 * _Z],
+    "tiny": [1e-160 * _X, 0.9 * _I],
+    "with a zero operator": [0.9 * _I, 0.0 * _X],
+    "nearly": [0.9 * _I, np.array([[0, 0.1], [0.1000001, 0]])],
+}
+
+
+@pytest.mark.parametrize("name", list(PAULI_CHANNELS))
+def test_pauli_channels_bit_exact(gpu, name):
+    """Channels of scaled Pauli operators (one pass with the gate before
+    them) and channels that only look like one, after 1-qubit, 2-qubit and
+    controlled gates, against the oracle's general sum."""
+    ops = [KrausOp(m) for m in PAULI_CHANNELS[name]]
+    for nm in (NoiseModel(Channel.custom(ops), None), NoiseModel(None, Channel.custom(ops)),
+               NoiseModel(Channel.custom(ops), Channel.bit_flip(0.1))):
+        for n in (1, 2, 4):
+            c = mixed_circuit(n, 31 * n)
+            want, _ = O.dm_run(c, nm.ev_struct())
+            got = DensityMatrixBackend.run_with_noise(c, nm).density_matrix().data()
+            assert np.array_equal(got, want), (name, n)
+        c = workloads.random_layers(7, 1, seed=3)
+        want, _ = O.dm_run(c, nm.ev_struct())
+        got = DensityMatrixBackend.run_with_noise(c, nm).density_matrix().data()
+        assert np.array_equal(got, want), name
+
+
 def test_observables_match_oracle(gpu):
     n = 5
     c = mixed_circuit(n, 77)
