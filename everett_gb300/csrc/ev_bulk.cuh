@@ -72,4 +72,22 @@ __device__ __forceinline__ void mbar_init_fence() {
   asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
 }
 
+// Asynchronous copy of one amplitude (8 or 16 bytes, naturally aligned) from
+// global to shared memory; copy_async_wait makes the calling thread's copies
+// visible to it (a barrier then makes them visible to the block).  16-byte
+// copies pass L1 by; 8-byte ones have no such form.
+template <typename V>
+__device__ __forceinline__ void copy_async(V* dst, const V* src) {
+  static_assert(sizeof(V) == 8 || sizeof(V) == 16, "amplitude size");
+  if constexpr (sizeof(V) == 16)
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_addr(dst)), "l"(src)
+                 : "memory");
+  else
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(smem_addr(dst)), "l"(src)
+                 : "memory");
+}
+__device__ __forceinline__ void copy_async_wait() {
+  asm volatile("cp.async.wait_all;" ::: "memory");
+}
+
 }  // namespace ev

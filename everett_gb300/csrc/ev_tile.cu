@@ -153,9 +153,13 @@ __global__ void __launch_bounds__(NT, MINB)
       }
       phase ^= 1;
     } else {
+      // asynchronous copies: all of a thread's share in flight at once and
+      // no registers held (loads into registers wait for one another: a
+      // store to the tile could alias the row offsets read next)
 #pragma unroll 4
-      for (uint32_t l = threadIdx.x; l < size; l += blockDim.x)
-        tile[l] = s[base | offs[l >> L] | (l & lowmask)];
+      for (uint32_t l = threadIdx.x; l < size; l += NT)
+        copy_async(tile + l, s + (base | offs[l >> L] | (l & lowmask)));
+      copy_async_wait();
       __syncthreads();
     }
     for (int o = 0; o < nops;) {
