@@ -46,6 +46,7 @@
 
 #include <sys/stat.h>
 
+#include "ev_stage.cuh"
 #include "ev_tile.cuh"
 
 namespace ev {
@@ -83,6 +84,13 @@ __device__ __forceinline__ uint32_t mat_words(uint8_t kind) {
   if (kind == T_DIAG2 || kind == T_DENSE2) return full;
   return 0;  // permutations, CZ, measurements, IfClassic prefixes
 }
+
+// complex64 circuits on tiles of 2^kStagedTile amplitudes and more run their
+// records in stages (ev_stage.cuh), smaller ones in sweeps and chains.  A
+// batch without such circuits takes the kernel compiled without stages, whose
+// fewer registers let three 256-thread CTAs share an SM (400 circuits of 4-9
+// qubits: 0.30 ms of device time with stages compiled in, 0.25 without).
+constexpr int kStagedTile = 11;
 
 struct BatchCirc {
   uint32_t n, k, npasses, pad;
@@ -143,18 +151,19 @@ __device__ bool wait_count(const unsigned* ctr, unsigned want) {
   return false;
 }
 
-template <typename V>
-__device__ __forceinline__ V ld_amp(const V* p, bool global) {
-  if (global) {
-    if constexpr (sizeof(V) == 16) {
-      const double2 v = __ldcg(reinterpret_cast<const double2*>(p));
-      return v;
-    } else {
-      const float2 v = __ldcg(reinterpret_cast<const float2*>(p));
-      return v;
-    }
-  }
-  return *p;
+// Where local amplitude l of a 2^k tile is stored (complex64 tiles are
+// swizzled for their stages).
+template <bool STAGES>
+__device__ __forceinline__ uint32_t tile_slot(uint32_t l, int k) {
+  return STAGES && k >= kStagedTile ? stage_slot(l) : l;
+}
+
+// Amplitude j of an n-qubit state in HBM (written by other CTAs: past L1) or
+// of a whole-state tile.
+template <bool STAGES, typename V>
+__device__ __forceinline__ V ld_amp(const V* p, uint64_t j, bool global, int n) {
+  if (global) return __ldcg(p + j);
+  return p[tile_slot<STAGES>(uint32_t(j), n)];
 }
 
 // Block-wide sum of two doubles (fixed tree shape).
@@ -178,14 +187,14 @@ __device__ void block_sum2(double* red, double& x, double& y) {
 // <Z_0>, sampling tree (level q at offset 2^q, as ev_sample builds it)
 // and shots of one circuit whose amplitudes are at `amps` (shared memory or
 // HBM).
-template <typename V>
+template <bool STAGES, typename V>
 __device__ void finalize(const V* amps, bool global, const BatchCirc& c, uint32_t ci, double* red,
                          const BatchArgs& a) {
   const int t = threadIdx.x, nb = blockDim.x;
   const uint64_t N = uint64_t(1) << c.n, half = N / 2;
   double r0 = 0.0, r1 = 0.0;
   for (uint64_t j = t; j < N; j += nb) {
-    const double p = nsq(ld_amp(amps + j, global));
+    const double p = nsq(ld_amp<STAGES>(amps, j, global, int(c.n)));
     if (j & 1)
       r1 += p;
     else
@@ -196,7 +205,7 @@ __device__ void finalize(const V* amps, bool global, const BatchCirc& c, uint32_
   double* tr = a.trees + c.tree;
   for (uint64_t r = t; r < half; r += nb)
     __stcg(tr + half + r,
-           __dadd_rn(nsq(ld_amp(amps + r, global)), nsq(ld_amp(amps + r + half, global))));
+           __dadd_rn(nsq(ld_amp<STAGES>(amps, r, global, int(c.n))), nsq(ld_amp<STAGES>(amps, r + half, global, int(c.n)))));
   __syncthreads();
   for (int q = int(c.n) - 2; q >= 0; --q) {
     const uint64_t w = uint64_t(1) << q;
@@ -210,7 +219,7 @@ __device__ void finalize(const V* amps, bool global, const BatchCirc& c, uint32_
     for (int q = 0; q < n; ++q) {
       const uint64_t w = uint64_t(1) << q;
       const double m = __ldcg(tr + w + r);
-      const double m1 = (q + 1 < n) ? __ldcg(tr + 2 * w + r + w) : nsq(ld_amp(amps + r + w, global));
+      const double m1 = (q + 1 < n) ? __ldcg(tr + 2 * w + r + w) : nsq(ld_amp<STAGES>(amps, r + w, global, int(c.n)));
       const double p1 = __ddiv_rn(m1, m);
       if (a.uni[c.uni + s * uint64_t(n) + q] < p1) r |= w;
     }
@@ -235,14 +244,14 @@ __device__ __forceinline__ V batch_scale(V a, double s) {
 // measure_qubit (measure.rs:15-51) on a whole state in shared memory: p1 by
 // a fixed block tree, the outcome from the circuit's next uniform, then the
 // collapse and rescale.  rng holds the circuit's xoshiro256++ state.
-template <typename V>
-__device__ void batch_measure(V* tile, uint32_t size, int q, uint32_t cbit, double* red,
+template <bool STAGES, typename V>
+__device__ void batch_measure(V* tile, int k, int q, uint32_t cbit, double* red,
                               uint8_t* cl, uint64_t* rng, double* meas) {
   const int t = threadIdx.x, nb = blockDim.x;
-  const uint32_t bit = 1u << q;
+  const uint32_t size = 1u << k, bit = 1u << q;
   double p1 = 0.0, unused = 0.0;
   for (uint32_t j = t; j < size; j += nb)
-    if (j & bit) p1 += nsq(tile[j]);
+    if (j & bit) p1 += nsq(tile[tile_slot<STAGES>(j, k)]);
   block_sum2(red, p1, unused);
   if (t == 0) {
     DevRng r(0);
@@ -261,16 +270,18 @@ __device__ void batch_measure(V* tile, uint32_t size, int q, uint32_t cbit, doub
   V zero;
   zero.x = 0;
   zero.y = 0;
-  for (uint32_t j = t; j < size; j += nb)
-    tile[j] = (((j & bit) != 0) == one) ? batch_scale(tile[j], scale) : zero;
+  for (uint32_t j = t; j < size; j += nb) {
+    V& a = tile[tile_slot<STAGES>(j, k)];
+    a = (((j & bit) != 0) == one) ? batch_scale(a, scale) : zero;
+  }
   __syncthreads();
 }
 
 // Compiled per block size: 256-thread CTAs, three of which fit an SM's
 // shared memory with the default tile, get 80 registers a thread; 512-thread
 // CTAs (two per SM) 64.
-template <typename V, int NT>
-__global__ void __launch_bounds__(NT, NT == 256 ? 3 : 2) k_batch(BatchArgs a, int kmax) {
+template <typename V, int NT, bool STAGES>
+__global__ void __launch_bounds__(NT, STAGES ? 512 / NT : NT == 256 ? 3 : 2) k_batch(BatchArgs a, int kmax) {
   extern __shared__ __align__(16) unsigned char sm[];
   V* tile = reinterpret_cast<V*>(sm);
   uint64_t* offs = reinterpret_cast<uint64_t*>(sm + (sizeof(V) << kmax));
@@ -309,7 +320,7 @@ __global__ void __launch_bounds__(NT, NT == 256 ? 3 : 2) k_batch(BatchArgs a, in
       if (!s_ok) continue;
     }
     if (it.kind == BI_FINAL) {
-      finalize(st, true, c, it.circ, red, a);
+      finalize<STAGES>(st, true, c, it.circ, red, a);
       __syncthreads();
       continue;
     }
@@ -336,7 +347,22 @@ __global__ void __launch_bounds__(NT, NT == 256 ? 3 : 2) k_batch(BatchArgs a, in
       for (uint32_t l = t; l < size; l += nb) tile[l] = z;
       if (t == 0 && base == 0) tile[0].x = 1;
     } else {
-      for (uint32_t l = t; l < size; l += nb) tile[l] = ld_amp(st + (base | offs[l >> L] | (l & lowmask)), true);
+      // groups of loads in flight before the first store (a store to the tile
+      // could alias the row offsets); past L1, other CTAs wrote the data
+      constexpr int G = sizeof(V) == 16 ? 4 : 8;
+      for (uint32_t l0 = t; l0 < size; l0 += G * NT) {
+        V v[G];
+#pragma unroll
+        for (int g = 0; g < G; ++g) {
+          const uint32_t l = l0 + uint32_t(g * NT);
+          if (l < size) v[g] = __ldcg(st + (base | offs[l >> L] | (l & lowmask)));
+        }
+#pragma unroll
+        for (int g = 0; g < G; ++g) {
+          const uint32_t l = l0 + uint32_t(g * NT);
+          if (l < size) tile[tile_slot<STAGES>(l, k)] = v[g];
+        }
+      }
     }
     __syncthreads();
     const PassRef pr = a.passes[c.pass0 + it.pass];
@@ -388,8 +414,15 @@ __global__ void __launch_bounds__(NT, NT == 256 ? 3 : 2) k_batch(BatchArgs a, in
         take = true;
         if (!go) continue;
         if (op.kind == B_MEAS) {
-          batch_measure(tile, size, op.p0, op.lmask, red, s_cl, s_rng, s_meas);
+          batch_measure<STAGES>(tile, k, op.p0, op.lmask, red, s_cl, s_rng, s_meas);
           continue;
+        }
+        if constexpr (STAGES) {
+          if (k >= kStagedTile) {
+            tile_stage(tile, k, rec, int(run), smat, base);
+            __syncthreads();
+            continue;
+          }
         }
         if ((base & op.emask) != op.emask) continue;
         if (run > 1 && op.ctype == CH_QUAD)
@@ -414,10 +447,10 @@ __global__ void __launch_bounds__(NT, NT == 256 ? 3 : 2) k_batch(BatchArgs a, in
       if constexpr (sizeof(V) == 16)
         __stcg(reinterpret_cast<double2*>(p), tile[l]);
       else
-        __stcg(reinterpret_cast<float2*>(p), tile[l]);
+        __stcg(reinterpret_cast<float2*>(p), tile[tile_slot<STAGES>(l, k)]);
     }
     if (it.kind == BI_WHOLE) {
-      finalize(tile, false, c, it.circ, red, a);
+      finalize<STAGES>(tile, false, c, it.circ, red, a);
     } else {
       __threadfence();
       __syncthreads();
@@ -548,6 +581,7 @@ void plan_circuit(const ev_circuit* c, int kmax, bool c64, uint32_t window, Circ
   const int k = n <= kmax ? n : kmax;
   out->k = k;
   const int L = std::min(k, 4);
+  const bool stages = c64 && k >= kStagedTile;
   out->classical = has_classical_ops(c);
   std::vector<Pass> passes;
   if (out->classical) {
@@ -591,9 +625,17 @@ void plan_circuit(const ev_circuit* c, int kmax, bool c64, uint32_t window, Circ
     recs.assign(p.ops.size(), TileOp{});
     for (size_t j = 0; j < p.ops.size(); ++j) {
       const ev_op& src = c->ops[p.ops[j]];
-      if (src.kind != EV_OP_MEASURE && src.kind != EV_OP_IF) encode_op(c, src, p.tset, local, &recs[j]);
+      if (src.kind == EV_OP_MEASURE || src.kind == EV_OP_IF) continue;
+      encode_op(c, src, p.tset, local, &recs[j]);
+      if (c64) pack_f32_matrix(recs[j].m, recs[j].kind == T_1Q ? 8 : 32);
+      if (stages && out->classical) mark_stages(&recs[j], 1, k, 1);
     }
-    if (!out->classical) mark_chains(recs.data(), recs.size(), chains, window);
+    if (!out->classical) {
+      if (stages)
+        mark_stages(recs.data(), recs.size(), k, window);
+      else
+        mark_chains(recs.data(), recs.size(), chains, window);
+    }
     for (size_t jj = 0; jj < p.ops.size(); ++jj) {
       const ev_op& src = c->ops[p.ops[jj]];
       if (src.kind == EV_OP_MEASURE || src.kind == EV_OP_IF) {
@@ -604,8 +646,7 @@ void plan_circuit(const ev_circuit* c, int kmax, bool c64, uint32_t window, Circ
         out->ops.push_back(b);
         continue;
       }
-      TileOp& tmp = recs[jj];
-      if (c64) pack_f32_matrix(tmp.m, tmp.kind == T_1Q ? 8 : 32);
+      const TileOp& tmp = recs[jj];
       BatchOp b;
       b.kind = tmp.kind;
       b.k1 = tmp.k1;
@@ -716,11 +757,14 @@ static int batch_once(Arena& A, const ev_batch_circuit* items, uint64_t count, i
   // shared memory: tile | row offsets | reduction scratch | staged records
   // and matrices.  The record window is as large as fits without costing a
   // resident CTA (at least 4 records).
-  const void* kfn = dtype == EV_C128
-                        ? (threads == 256 ? reinterpret_cast<const void*>(k_batch<double2, 256>)
-                                          : reinterpret_cast<const void*>(k_batch<double2, 512>))
-                        : (threads == 256 ? reinterpret_cast<const void*>(k_batch<float2, 256>)
-                                          : reinterpret_cast<const void*>(k_batch<float2, 512>));
+  bool stages = false;
+  for (uint64_t i = 0; i < count && dtype == EV_C64; ++i)
+    stages = stages || std::min(int(items[i].circuit.num_qubits), kmax) >= kStagedTile;
+  void (*const kernel)(BatchArgs, int) =
+      dtype == EV_C128 ? (threads == 256 ? k_batch<double2, 256, false> : k_batch<double2, 512, false>)
+      : stages         ? (threads == 256 ? k_batch<float2, 256, true> : k_batch<float2, 512, true>)
+                       : (threads == 256 ? k_batch<float2, 256, false> : k_batch<float2, 512, false>);
+  const void* kfn = reinterpret_cast<const void*>(kernel);
   EV_TRY(prepare_smem_kernel(kfn));
   const size_t smem_base =
       ((ab << kmax) + (size_t(8) << (kmax > 4 ? kmax - 4 : 0)) + 2 * size_t(threads) * 8 + 15) &
@@ -886,14 +930,7 @@ static int batch_once(Arena& A, const ev_batch_circuit* items, uint64_t count, i
   if (debug_enabled())
     fprintf(stderr, "[ev] k_batch dtype %d tile %d threads %d smem %zu window %u: %d CTAs/SM, %zu items\n",
             dtype, kmax, threads, smem, window, per_sm, q.size());
-  if (dtype == EV_C128 && threads == 256)
-    k_batch<double2, 256><<<grid, threads, smem, A.stream>>>(args, kmax);
-  else if (dtype == EV_C128)
-    k_batch<double2, 512><<<grid, threads, smem, A.stream>>>(args, kmax);
-  else if (threads == 256)
-    k_batch<float2, 256><<<grid, threads, smem, A.stream>>>(args, kmax);
-  else
-    k_batch<float2, 512><<<grid, threads, smem, A.stream>>>(args, kmax);
+  kernel<<<grid, threads, smem, A.stream>>>(args, kmax);
   EV_CUDA(cudaGetLastError());
   EV_CUDA(cudaEventRecord(A.e1, A.stream));
   // results: shots | expz, one copy down
@@ -1027,7 +1064,10 @@ extern "C" int ev_batch_run(const ev_batch_circuit* items, uint64_t count, const
     }
   }
   if (kbits <= 0) kbits = default_tile_bits_batch(dtype);
-  if (threads <= 0) threads = 512;
+  // complex64: two CTAs of 256 threads keep the 16 amplitudes of a stage in
+  // 128 registers a thread (512 circuits of 8-18 qubits: 12.3 ms of device
+  // time against 14.2 with one CTA of 512)
+  if (threads <= 0) threads = dtype == EV_C64 ? 256 : 512;
   if (kbits > kcap) kbits = kcap;
   if (kbits < 4) kbits = 4;
   if (threads != 256 && threads != 512)

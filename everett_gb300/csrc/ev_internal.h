@@ -156,6 +156,10 @@ struct TilePlan {
 struct SegStep {
   int fused = 0;        // 0: tile pass, 1: fused unitary
   TilePlan tile{};      // tile: its qubits
+  int threads = 0;      // tile: threads per block and blocks per SM (the
+  int per_sm = 0;       // records are laid out for them)
+  int bulk = 0;         // tile: moved by the bulk-copy engine
+  int stages = 0;       // complex64 tile: records in stages (ev_stage.cuh)
   size_t off0 = 0;      // fused: FusedDesc offset (in the blob)
   size_t off1 = 0;      // tile: first op record; fused: matrix operands
   int nops = 0;         // tile: op records

@@ -19,6 +19,7 @@
 #include <cstring>
 
 #include "ev_bulk.cuh"
+#include "ev_stage.cuh"
 #include "ev_tile.cuh"
 
 namespace ev {
@@ -83,11 +84,12 @@ constexpr uint32_t kTileWaitLimit = 1u << 24;  // try_wait polls before giving u
 // block: [tile 2^k amplitudes][row offsets 2^(k-L)][op records][comp qubits].
 // A load that never completes sets *err (the run's device flag, reported as
 // EV_ERR_TIMEOUT) and ends the block after a bounded drain.
-template <typename V, bool BULK, int NT, int MINB>
+template <typename V, bool BULK, int NT, int MINB, bool STAGES>
 __global__ void __launch_bounds__(NT, MINB)
     k_tile(V* __restrict__ s, uint64_t ntiles, const __grid_constant__ TilePlan plan,
            const TileOp* __restrict__ gops, int nops, int* err) {
   constexpr bool kStageOps = !(NT == 256 && MINB == 3);
+  static_assert(!STAGES || (sizeof(V) == 8 && !BULK), "complex64, plain copies");
   // the next pass may start its own staging now; it waits below for this one
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -158,14 +160,17 @@ __global__ void __launch_bounds__(NT, MINB)
       // store to the tile could alias the row offsets read next)
 #pragma unroll 4
       for (uint32_t l = threadIdx.x; l < size; l += NT)
-        copy_async(tile + l, s + (base | offs[l >> L] | (l & lowmask)));
+        copy_async(tile + (STAGES ? stage_slot(l) : l), s + (base | offs[l >> L] | (l & lowmask)));
       copy_async_wait();
       __syncthreads();
     }
     for (int o = 0; o < nops;) {
       const TileOp& op = ops[o];
       const int run = op.run > 1 ? op.run : 1;
-      if ((base & op.emask) == op.emask) {  // uniform across the block
+      if constexpr (STAGES) {
+        tile_stage(tile, k, ops + o, run, nullptr, base);
+        __syncthreads();
+      } else if ((base & op.emask) == op.emask) {  // uniform across the block
         if (run > 1 && op.ctype == CH_QUAD)
           tile_quad_chain(tile, size, ops + o, run, nullptr);
         else if (run > 1 && op.ctype == CH_DIAG)
@@ -192,21 +197,21 @@ __global__ void __launch_bounds__(NT, MINB)
     } else {
 #pragma unroll 4
       for (uint32_t l = threadIdx.x; l < size; l += blockDim.x)
-        s[base | offs[l >> L] | (l & lowmask)] = tile[l];
+        s[base | offs[l >> L] | (l & lowmask)] = tile[STAGES ? stage_slot(l) : l];
     }
     __syncthreads();
   }
   if (use_bulk && warp == 0) bulk_wait_all();
 }
 
-template <typename V, bool BULK, int NT, int MINB>
+template <typename V, bool BULK, int NT, int MINB, bool STAGES = false>
 static int launch_tile_as(ev_state* s, uint64_t ntiles, size_t smem, const TilePlan& plan,
                           const TileOp* dops, int nops) {
-  EV_TRY(prepare_smem_kernel(reinterpret_cast<const void*>(k_tile<V, BULK, NT, MINB>)));
+  EV_TRY(prepare_smem_kernel(reinterpret_cast<const void*>(k_tile<V, BULK, NT, MINB, STAGES>)));
   uint64_t grid = ntiles;
   if (ntiles > uint64_t(s->num_sms)) {
     int per_sm = 0;
-    EV_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_tile<V, BULK, NT, MINB>, NT,
+    EV_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_tile<V, BULK, NT, MINB, STAGES>, NT,
                                                           smem));
     if (per_sm < 1) per_sm = 1;
     grid = std::min(ntiles, uint64_t(s->num_sms) * per_sm);
@@ -230,32 +235,54 @@ static int launch_tile_as(ev_state* s, uint64_t ntiles, size_t smem, const TileP
   // qubits, 128 blocks, 0.85 / 0.68; 20 qubits, 304 blocks of 256 threads,
   // 8.50 / 7.20).
   cfg.numAttrs = 2 * grid <= uint64_t(s->num_sms) ? 1 : 0;
-  EV_CUDA(cudaLaunchKernelEx(&cfg, k_tile<V, BULK, NT, MINB>, static_cast<V*>(s->amps), ntiles,
+  EV_CUDA(cudaLaunchKernelEx(&cfg, k_tile<V, BULK, NT, MINB, STAGES>, static_cast<V*>(s->amps), ntiles,
                              plan, dops, nops, derr));
   return EV_OK;
 }
 
-// Threads of a block: one per pair of a tile of up to 2^8 amplitudes, one per
-// quad above.
-static int tile_block(int k) { return k <= 9 ? 128 : k <= 11 ? 256 : kTileThreads; }
+// Block shape of a pass over tiles of 2^k amplitudes, and whether its
+// complex64 records run in stages (tile_shape and the bulk-copy mover
+// override it).
+static void choose_block(int dtype, int k, SegStep* st) {
+  st->bulk = tile_bulk_enabled() ? 1 : 0;
+  const int shape = st->bulk ? 0 : tile_shape();
+  if (shape == 1) {
+    st->threads = 256;
+    st->per_sm = 3;
+  } else if (shape == 2) {
+    st->threads = kTileThreads;
+    st->per_sm = 1;
+  } else if (!st->bulk && k <= 11) {
+    st->threads = k <= 9 ? 128 : 256;
+    st->per_sm = k <= 9 ? 4 : 2;
+  } else if (!st->bulk && dtype == EV_C64) {
+    st->stages = 1;
+    st->threads = 256;
+    st->per_sm = 2;
+  } else {
+    st->threads = kTileThreads;
+    st->per_sm = 2;
+  }
+}
 
 template <typename V>
-static int launch_tile(ev_state* s, uint64_t ntiles, const TilePlan& plan, const TileOp* dops,
-                       int nops) {
+static int launch_tile(ev_state* s, const SegStep& st, const TileOp* dops) {
+  const TilePlan& plan = st.tile;
   const size_t ops_at = (sizeof(V) * (size_t(1) << plan.k) +
                          sizeof(uint64_t) * (size_t(1) << (plan.k - plan.L)) + 15) & ~size_t(15);
-  const bool bulk = tile_bulk_enabled();
-  const int shape = tile_shape();
-  if (shape == 1 && !bulk)
-    return launch_tile_as<V, false, 256, 3>(s, ntiles, ops_at + 64, plan, dops, nops);
-  const size_t smem = ops_at + sizeof(TileOp) * size_t(nops) + 64;
-  if (shape == 2 && !bulk)
-    return launch_tile_as<V, false, kTileThreads, 1>(s, ntiles, smem, plan, dops, nops);
-  if (bulk) return launch_tile_as<V, true, kTileThreads, 2>(s, ntiles, smem, plan, dops, nops);
-  const int threads = tile_block(plan.k);
-  if (threads == 128) return launch_tile_as<V, false, 128, 4>(s, ntiles, smem, plan, dops, nops);
-  if (threads == 256) return launch_tile_as<V, false, 256, 2>(s, ntiles, smem, plan, dops, nops);
-  return launch_tile_as<V, false, kTileThreads, 2>(s, ntiles, smem, plan, dops, nops);
+  const size_t smem = ops_at + sizeof(TileOp) * size_t(st.nops) + 64;
+  const int n = st.nops;
+  if (st.bulk) return launch_tile_as<V, true, kTileThreads, 2>(s, st.count, smem, plan, dops, n);
+  if constexpr (sizeof(V) == 8)
+    if (st.stages) return launch_tile_as<V, false, 256, 2, true>(s, st.count, smem, plan, dops, n);
+  switch (st.threads + st.per_sm) {
+    case 128 + 4: return launch_tile_as<V, false, 128, 4>(s, st.count, smem, plan, dops, n);
+    case 256 + 2: return launch_tile_as<V, false, 256, 2>(s, st.count, smem, plan, dops, n);
+    case 256 + 3:  // its records are read through L1
+      return launch_tile_as<V, false, 256, 3>(s, st.count, ops_at + 64, plan, dops, n);
+    case 512 + 1: return launch_tile_as<V, false, 512, 1>(s, st.count, smem, plan, dops, n);
+    default: return launch_tile_as<V, false, 512, 2>(s, st.count, smem, plan, dops, n);
+  }
 }
 
 // Tile bits when the caller names none.  A complex128 pass is bound by the
@@ -266,15 +293,14 @@ static int launch_tile(ev_state* s, uint64_t ntiles, const TilePlan& plan, const
 // random-layer circuit (depth 10 at 10 qubits), tiles of 2^8 / 2^10 / 2^12:
 // 10 qubits 0.21 / 0.41 / -; 14 qubits 0.61 / 1.09 / 2.94; 17 qubits
 // 1.10 / 1.82 / 3.60; 18 qubits 2.24 / 2.00 / 5.5; 19 qubits 4.2 / 4.1 /
-// 4.0; 20 qubits 8.4 / 8.5 / 7.4.  complex64 (2^8 / 2^10 / 2^12 / 2^13): 14
-// qubits 0.22 / 0.24 / 0.45 / 0.76; 17 qubits 0.33 / 0.38 / 0.56 / 0.95; 18
-// qubits 0.56 / 0.43 / 0.70 / 0.99; 20 qubits 1.6 / 1.2 / 0.92 / 1.54; 22
-// qubits, depth 10, 3.3 / 2.0 / 1.9 / 1.7.
+// 4.0; 20 qubits 8.4 / 8.5 / 7.4.  complex64 (2^8 / 2^10 / 2^12 / 2^13, the
+// last two in stages): 14 qubits 0.21 / 0.23 / 0.38 / 0.66; 17 qubits 0.36 /
+// 0.32 / 0.47 / 0.82; 18 qubits 0.62 / 0.40 / 0.55 / 0.87; 20 qubits - / 1.30
+// / 0.85 / 1.08; 22 qubits, depth 10, - / 2.5 / 1.39 / 1.49; 25-qubit QFT - /
+// 12.9 / 3.5 / 3.2.
 int default_tile_bits(int dtype, int n) {
-  if (n <= 17) return 8;
-  if (n <= 18) return 10;
-  if (dtype == EV_C128) return 12;
-  return n <= 19 ? 10 : n <= 20 ? 12 : 13;
+  if (dtype == EV_C128) return n <= 17 ? 8 : n <= 18 ? 10 : 12;
+  return n <= 15 ? 8 : n <= 19 ? 10 : n <= 22 ? 12 : 13;
 }
 
 // Plans a gate run into tile passes; plans and records go into the blob.
@@ -299,7 +325,9 @@ int plan_tiled(ev_state* s, const ev_circuit* c, uint64_t first, uint64_t last, 
   const SoftLevels soft = tile_soft_levels();
   // a quad chain occupies a thread per four amplitudes: where that leaves
   // threads idle, pair chains finish sooner (14 qubits 0.94 -> 0.61 ms)
-  const bool quads = (1 << k) / 4 >= tile_block(k);
+  SegStep shape;
+  choose_block(s->dtype, k, &shape);
+  const bool quads = (1 << k) / 4 >= shape.threads;
   const ChainSet chains = chain_set("EV_TILE_CHAIN", ChainSet{true, quads, true});
   std::vector<TileOp> ops;
   for (const Pass& p : passes) {
@@ -324,9 +352,11 @@ int plan_tiled(ev_state* s, const ev_circuit* c, uint64_t first, uint64_t last, 
       if (s->dtype == EV_C128 && ops[j].kind == T_1Q)
         ops[j].soft = uint8_t(ops[j].k1 == K1_REAL ? soft.real : soft.other);
     }
-    mark_chains(ops.data(), ops.size(), chains);
-    SegStep st;
-    st.fused = 0;
+    if (shape.stages)
+      mark_stages(ops.data(), ops.size(), k, 255);
+    else
+      mark_chains(ops.data(), ops.size(), chains);
+    SegStep st = shape;
     st.tile = plan;
     st.off1 = blob->add(ops.data(), ops.size() * sizeof(TileOp));
     st.nops = int(ops.size());
@@ -338,8 +368,7 @@ int plan_tiled(ev_state* s, const ev_circuit* c, uint64_t first, uint64_t last, 
 
 int launch_tile_step(ev_state* s, const SegStep& st, const unsigned char* dblob) {
   const TileOp* dops = reinterpret_cast<const TileOp*>(dblob + st.off1);
-  if (s->dtype == EV_C128) return launch_tile<double2>(s, st.count, st.tile, dops, st.nops);
-  return launch_tile<float2>(s, st.count, st.tile, dops, st.nops);
+  return s->dtype == EV_C128 ? launch_tile<double2>(s, st, dops) : launch_tile<float2>(s, st, dops);
 }
 
 // ---- device check of the integer-pipe product ------------------------------------

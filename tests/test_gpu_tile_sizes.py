@@ -63,3 +63,45 @@ def test_default_tiles_replayed(gpu, dtype):
         assert prepared.launch(9) == st.classical()
         assert np.array_equal(again.amplitudes(), st.state().amplitudes())
     prepared.close()
+
+
+def every_record_kind(n, seed, count):
+    """1-qubit kinds (real, Rx-like, dense, diagonal, phase, anti-diagonal,
+    identity) free and under one to three controls, CNOT, CZ, SWAP, parity
+    and general diagonals and a dense 4x4, on random positions."""
+    rng = np.random.default_rng(seed)
+    ones = [Gate1.h(), Gate1.ry(0.4), Gate1.rx(0.7), Gate1.rz(1.1), Gate1.phase(0.9), Gate1.t(),
+            Gate1.x(), Gate1.y(), Gate1.z(), Gate1.id(),
+            Gate1(0.6 + 0.1j, -0.3 + 0.2j, 0.25 - 0.7j, 0.1 + 0.05j)]
+    unit = np.exp(1j * rng.uniform(0, 6, 4))
+    twos = [Gate2.cnot(), Gate2.cz(), Gate2.swap(), Gate2.rzz(0.8), Gate2(np.diag(unit)),
+            Gate2(np.linalg.qr(rng.normal(size=(4, 4)) + 1j * rng.normal(size=(4, 4)))[0])]
+    c = Circuit(n)
+    for q in range(n):
+        c.h(q)
+    for _ in range(count):
+        q = [int(v) for v in rng.choice(n, 4, replace=False)]
+        k = int(rng.integers(0, 3))
+        if k == 0:
+            c.gate1(ones[int(rng.integers(len(ones)))], q[0])
+        elif k == 1:
+            c.controlled(q[1:2 + int(rng.integers(3))], ones[int(rng.integers(len(ones)))], q[0])
+        else:
+            c.gate2(twos[int(rng.integers(len(twos)))], q[0], q[1])
+    return c
+
+
+@pytest.mark.parametrize("n,tile_bits", [(12, 12), (13, 13), (14, 14), (15, 12), (16, 13)])
+def test_stages_equal_sweeps(gpu, monkeypatch, n, tile_bits):
+    """complex64 records in stages (16 amplitudes a thread in registers)
+    against one sweep per record on the same tiles (the 256-thread block
+    shape): each amplitude sees the same operations in the same order, so the
+    bits agree; and the oracle's amplitudes to the complex64 bar."""
+    c = every_record_kind(n, 100 * n + tile_bits, 400)
+    staged = CudaStateVectorBackend.run(c, dtype="complex64", tile_bits=tile_bits).state().amplitudes()
+    monkeypatch.setenv("EV_TILE_THREADS", "256")
+    swept = CudaStateVectorBackend.run(c, dtype="complex64", tile_bits=tile_bits).state().amplitudes()
+    assert np.array_equal(staged, swept)
+    want, _, _ = O.run_seeded(c, 0, parallel=True)
+    want = want / np.linalg.norm(want)
+    assert np.max(np.abs(staged - want)) < 1e-5
