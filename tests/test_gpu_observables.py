@@ -141,3 +141,23 @@ def test_many_groups_from_one_read(gpu, n, dtype):
         xm, zm = p.masks()
         want = O.pauli_expectation(ref, xm, zm, p.neg)
         assert abs(g - want) < 1e-12, (n, dtype, str(p), g, want)
+
+
+def test_marginal_low_complex64_bits(gpu):
+    """complex64 marginals square each part exactly on the integer pipes: the
+    f64 sums of the exact squares in basis order, for zero, subnormal, tiny,
+    ordinary and huge parts and odd numbers of terms per bin."""
+    rng = np.random.default_rng(3)
+    n = 11
+    a = (rng.normal(size=1 << n) * 10.0 ** rng.integers(-44, 38, 1 << n)).astype(np.float32)
+    b = (rng.normal(size=1 << n) * 10.0 ** rng.integers(-44, 38, 1 << n)).astype(np.float32)
+    a[:40], b[20:60] = 0.0, 0.0
+    amps = a.astype(np.complex128) + 1j * b.astype(np.complex128)
+    st = State.from_amplitudes(amps, dtype="complex64")
+    x, y = a.astype(np.float64), b.astype(np.float64)
+    terms = x * x + y * y  # both squares are exact in f64
+    for m in (0, 3, 8, 10, 11):
+        want = np.zeros(1 << m)
+        for row in terms.reshape(-1, 1 << m):
+            want = want + row
+        assert np.array_equal(st.marginal_low(m), want), m
