@@ -73,6 +73,20 @@ def test_batch_c64_fidelity_and_shots(gpu, threads):
         assert np.array_equal(r.shots, O.sample_tree(np.ascontiguousarray(got), i, 200))
 
 
+@pytest.mark.parametrize("n,shots", [(1, 1), (3, 85), (4, 64), (5, 103), (2, 32768), (3, 21846),
+                                     (7, 30000)])
+def test_batch_shot_uniforms_across_chunks(gpu, n, shots):
+    """The shot uniforms are drawn in chunks of 256 by many threads (256
+    chunks a block): draw counts at and around one chunk, one block and
+    several blocks give the shots of the sequential stream."""
+    c = workloads.random_layers(n, 2, seed=n)
+    want, _, _ = O.run_seeded(c, 0)
+    res, _ = batch.run_batch([c, c], seeds=[11, 2**63 + 5], shots=[shots, max(1, shots // 3)],
+                             dtype="complex128")
+    for r, seed, k in zip(res, (11, 2**63 + 5), (shots, max(1, shots // 3))):
+        assert np.array_equal(r.shots, O.sample_tree(want, seed, k))
+
+
 def test_batch_matches_single_runs(gpu):
     """A circuit gives the same final state alone and inside a batch."""
     circs = tfim_mix(12, 4, 14, seed=3)
