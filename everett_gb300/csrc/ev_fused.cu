@@ -339,6 +339,21 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t v[16]) {
       : "r"(taddr));
 }
 
+__device__ __forceinline__ void tmem_st8(uint32_t taddr, const float v[8]) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};\n" ::"r"(taddr),
+               "f"(v[0]), "f"(v[1]), "f"(v[2]), "f"(v[3]), "f"(v[4]), "f"(v[5]), "f"(v[6]), "f"(v[7])
+               : "memory");
+}
+
+// D += A B with A (128 rows, one 32-bit element per column) in TMEM.
+__device__ __forceinline__ void mma_tf32_ta(uint32_t dtmem, uint32_t atmem, uint64_t b,
+                                            uint32_t idesc, uint32_t acc) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::tf32 [%0], [%1], %2, %3, p;\n\t}\n" ::"r"(dtmem),
+      "r"(atmem), "l"(b), "r"(idesc), "r"(acc));
+}
+
 template <int VAR>
 struct Elem;
 template <>
@@ -386,6 +401,15 @@ struct TcShape {
   static constexpr int B_BYTES = K * K * ESZ;
   static constexpr int SMEM = 2 * A_BYTES + 2 * B_BYTES + 1024 /* align */ + 64;
   static constexpr int TMEM_COLS = K < 32 ? 32 : K;
+  // k_fused_tc: TF32 keeps the high parts of A in TMEM, in the K columns
+  // above the accumulator.  They are read by two of the three products, and
+  // without them a CTA takes 65 KiB of shared memory instead of 97: three
+  // CTAs per SM instead of two (28 qubits: 996 us a pass, 816 now,
+  // 642 at the copy bandwidth).
+  static constexpr bool kHiInTmem = VAR == EV_FUSED_TF32X3;
+  static constexpr int TC_SMEM = SMEM - (kHiInTmem ? A_BYTES : 0);
+  static constexpr int TC_TMEM_COLS = kHiInTmem ? 2 * K : TMEM_COLS;
+  static constexpr int TC_CTAS = kHiInTmem ? 3 : KB == 5 ? 4 : 2;  // resident per SM
 };
 
 constexpr uint32_t kWaitLimit = 1u << 24;
@@ -393,7 +417,7 @@ constexpr uint32_t kWaitLimit = 1u << 24;
 constexpr int kTcThreads = 256;  // 8 warps: warps w and w+4 share TMEM lane quarter w
 
 template <int KB, int VAR>
-__global__ void __launch_bounds__(kTcThreads)
+__global__ void __launch_bounds__(kTcThreads, TcShape<KB, VAR>::TC_CTAS)
     k_fused_tc(float2* __restrict__ s, const FusedDesc* __restrict__ gd,
                const unsigned char* __restrict__ bmat, int* __restrict__ err) {
   using Sh = TcShape<KB, VAR>;
@@ -404,10 +428,10 @@ __global__ void __launch_bounds__(kTcThreads)
   __shared__ uint32_t tmem_slot;
   unsigned char* sm = reinterpret_cast<unsigned char*>(
       (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  unsigned char* a_hi = sm;
-  unsigned char* a_lo = sm + Sh::A_BYTES;
-  unsigned char* b_hi = sm + 2 * Sh::A_BYTES;
+  unsigned char* a_lo = sm;
+  unsigned char* b_hi = sm + Sh::A_BYTES;
   unsigned char* b_lo = b_hi + Sh::B_BYTES;
+  [[maybe_unused]] unsigned char* a_hi = b_lo + Sh::B_BYTES;
   const int tid = threadIdx.x, warp = tid >> 5;
 
   for (int i = tid; i < int(sizeof(FusedDesc) / 8); i += blockDim.x)
@@ -432,7 +456,7 @@ __global__ void __launch_bounds__(kTcThreads)
   if (warp == 0) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
                      smem_addr(&tmem_slot)),
-                 "r"(uint32_t(Sh::TMEM_COLS)));
+                 "r"(uint32_t(Sh::TC_TMEM_COLS)));
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
   }
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -458,6 +482,7 @@ __global__ void __launch_bounds__(kTcThreads)
   const uint32_t rsw = uint32_t((row >> 3) * 1024 + (row & 7) * 128);
   const uint32_t rx = uint32_t(row & 7);
   const uint64_t roff = d.rtab[row];
+  const uint32_t lane_tmem = tmem + (uint32_t(quarter * 32) << 16);
   // L2 prefetch of the rows two steps ahead: contiguous runs of 2^lowbits
   // amplitudes, one bulk prefetch per run from warp 1
   const int nruns = 1 << (d.k + 7 - d.lowbits);
@@ -494,8 +519,7 @@ __global__ void __launch_bounds__(kTcThreads)
           lo[2 * i + 1] = im - hi[2 * i + 1];
         }
         const uint32_t o0 = kb + (((c0) ^ rx) << 4), o1 = kb + (((c0 + 1) ^ rx) << 4);
-        *reinterpret_cast<float4*>(a_hi + o0) = make_float4(hi[0], hi[1], hi[2], hi[3]);
-        *reinterpret_cast<float4*>(a_hi + o1) = make_float4(hi[4], hi[5], hi[6], hi[7]);
+        tmem_st8(lane_tmem + uint32_t(K + 8 * g), hi);
         *reinterpret_cast<float4*>(a_lo + o0) = make_float4(lo[0], lo[1], lo[2], lo[3]);
         *reinterpret_cast<float4*>(a_lo + o1) = make_float4(lo[4], lo[5], lo[6], lo[7]);
       } else {
@@ -516,10 +540,15 @@ __global__ void __launch_bounds__(kTcThreads)
       }
     }
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    if constexpr (Sh::kHiInTmem) {
+      asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    }
     __syncthreads();
     if (tid == 0) {
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      const uint32_t ah = smem_addr(a_hi), al = smem_addr(a_lo);
+      [[maybe_unused]] const uint32_t ah = smem_addr(a_hi);
+      const uint32_t al = smem_addr(a_lo);
       const uint32_t bh = smem_addr(b_hi), bl = smem_addr(b_lo);
       constexpr int per_row = 128 / ESZ;
       uint32_t acc = 0;
@@ -529,9 +558,14 @@ __global__ void __launch_bounds__(kTcThreads)
         const uint32_t kin = uint32_t((kk % per_row) * ESZ);
         const uint32_t ao = uint32_t(kb * kRows * 128) + kin;
         const uint32_t bo = uint32_t(kb * K * 128) + kin;
-        mma_issue<VAR>(tmem, sw128_desc(ah + ao), sw128_desc(bh + bo), idesc, acc);
+        if constexpr (Sh::kHiInTmem) {
+          mma_tf32_ta(tmem, tmem + uint32_t(K + kk), sw128_desc(bh + bo), idesc, acc);
+          mma_tf32_ta(tmem, tmem + uint32_t(K + kk), sw128_desc(bl + bo), idesc, 1);
+        } else {
+          mma_issue<VAR>(tmem, sw128_desc(ah + ao), sw128_desc(bh + bo), idesc, acc);
+          mma_issue<VAR>(tmem, sw128_desc(ah + ao), sw128_desc(bl + bo), idesc, 1);
+        }
         acc = 1;
-        mma_issue<VAR>(tmem, sw128_desc(ah + ao), sw128_desc(bl + bo), idesc, 1);
         mma_issue<VAR>(tmem, sw128_desc(al + ao), sw128_desc(bh + bo), idesc, 1);
       }
       asm volatile(
@@ -546,12 +580,11 @@ __global__ void __launch_bounds__(kTcThreads)
     }
     phase ^= 1;
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    const uint32_t lane_base = tmem + (uint32_t(quarter * 32) << 16);
     const bool pair_store = d.ftab[1] == 1;  // f bit 0 is qubit 0: outputs a, a+1 adjacent
 #pragma unroll
     for (int c0 = half * (K / 2); c0 < (half + 1) * (K / 2); c0 += 16) {
       uint32_t w[16];
-      tmem_ld16(lane_base + uint32_t(c0), w);
+      tmem_ld16(lane_tmem + uint32_t(c0), w);
       asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
       if (pair_store) {
 #pragma unroll
@@ -576,7 +609,7 @@ __global__ void __launch_bounds__(kTcThreads)
   __syncthreads();
   if (warp == 0) {
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem),
-                 "r"(uint32_t(Sh::TMEM_COLS)));
+                 "r"(uint32_t(Sh::TC_TMEM_COLS)));
   }
 }
 
@@ -1354,22 +1387,22 @@ static int launch_tc(ev_state* s, const FusedDesc* dd, const unsigned char* db, 
   EV_CUDA(cudaFuncGetAttributes(&fa, k_fused_tc<KB, VAR>));
   int smem_sm = 0;
   EV_CUDA(cudaDeviceGetAttribute(&smem_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, s->device));
-  int per_sm = smem_sm / int(Sh::SMEM + fa.sharedSizeBytes + 1024);
+  int per_sm = smem_sm / int(Sh::TC_SMEM + fa.sharedSizeBytes + 1024);
   int regs_sm = 0;
   EV_CUDA(cudaDeviceGetAttribute(&regs_sm, cudaDevAttrMaxRegistersPerMultiprocessor, s->device));
   const int by_regs = regs_sm / ((fa.numRegs + 7) / 8 * 8 * kTcThreads);
   if (per_sm > by_regs) per_sm = by_regs;
   if (per_sm < 1) per_sm = 1;
   // keep every resident CTA's TMEM allocation satisfiable at once
-  const int tmem_cap = 512 / Sh::TMEM_COLS;
+  const int tmem_cap = 512 / Sh::TC_TMEM_COLS;
   if (per_sm > tmem_cap) per_sm = tmem_cap;
   s->tc_ctas_per_sm = per_sm;
   uint64_t grid = uint64_t(s->num_sms) * per_sm;
   if (grid > nsteps) grid = nsteps;
   if (debug_enabled())
     fprintf(stderr, "[ev] k_fused_tc<%d,%d> smem %d+%zu per CTA, %d CTAs/SM, grid %llu\n", KB, VAR,
-            Sh::SMEM, size_t(fa.sharedSizeBytes), per_sm, (unsigned long long)grid);
-  k_fused_tc<KB, VAR><<<unsigned(grid), kTcThreads, Sh::SMEM, s->stream>>>(
+            Sh::TC_SMEM, size_t(fa.sharedSizeBytes), per_sm, (unsigned long long)grid);
+  k_fused_tc<KB, VAR><<<unsigned(grid), kTcThreads, Sh::TC_SMEM, s->stream>>>(
       static_cast<float2*>(s->amps), dd, db, derr);
   EV_CUDA(cudaGetLastError());
   return EV_OK;
