@@ -78,55 +78,73 @@ struct Block {
   std::vector<cd> U;            // 2^k x 2^k row-major
 };
 
-static void op_qubits(const ev_circuit* c, const ev_op& op, std::vector<int>* q) {
-  q->clear();
-  if (op.kind == EV_OP_APPLY2) {
-    q->push_back(int(op.q0));
-    q->push_back(int(op.q1));
-    return;
-  }
-  q->push_back(int(op.q0));
+static uint64_t op_qubits(const ev_circuit* c, const ev_op& op) {
+  uint64_t m = uint64_t(1) << op.q0;
+  if (op.kind == EV_OP_APPLY2) return m | uint64_t(1) << op.q1;
   if (op.kind == EV_OP_CONTROLLED)
-    for (uint32_t j = 0; j < op.nctrl; ++j) {
-      const int cq = int(c->ctrl_pool[op.ctrl_off + j]);
-      if (std::find(q->begin(), q->end(), cq) == q->end()) q->push_back(cq);
-    }
+    for (uint32_t j = 0; j < op.nctrl; ++j) m |= uint64_t(1) << c->ctrl_pool[op.ctrl_off + j];
+  return m;
 }
 
-// Left-multiplies U (d x d, local bit i <-> F[i]) by one gate record.
+// The planner's complex arithmetic, written out on rows of interleaved
+// doubles: std::complex multiplies through a library call that checks for
+// NaN, which made fusing the blocks of a 16-qubit run take longer than
+// running them.
+// (x, y) <- (m0 x + m1 y, m2 x + m3 y) over two rows of n complex values
+static void mix_rows(const double* m, double* x, double* y, int n) {
+  for (int i = 0; i < 2 * n; i += 2) {
+    const double xr = x[i], xi = x[i + 1], yr = y[i], yi = y[i + 1];
+    x[i] = (m[0] * xr - m[1] * xi) + (m[2] * yr - m[3] * yi);
+    x[i + 1] = (m[0] * xi + m[1] * xr) + (m[2] * yi + m[3] * yr);
+    y[i] = (m[4] * xr - m[5] * xi) + (m[6] * yr - m[7] * yi);
+    y[i + 1] = (m[4] * xi + m[5] * xr) + (m[6] * yi + m[7] * yr);
+  }
+}
+
+// Left-multiplies U (d x d, local bit i <-> F[i]) by one gate record: the
+// gate combines whole rows of U.
 static void apply_to_unitary(const ev_circuit* c, const ev_op& op, const std::vector<int>& F,
                              std::vector<cd>* U) {
   const int d = int(1u << F.size());
-  auto loc = [&](int q) { return int(std::find(F.begin(), F.end(), q) - F.begin()); };
-  auto m = [&](int i) { return cd(op.m[2 * i], op.m[2 * i + 1]); };
+  auto loc = [&](uint64_t q) { return int(std::find(F.begin(), F.end(), int(q)) - F.begin()); };
+  auto row = [&](int r) { return reinterpret_cast<double*>(U->data() + size_t(r) * d); };
   if (op.kind == EV_OP_APPLY2) {
-    const int ba = 1 << loc(int(op.q0)), bb = 1 << loc(int(op.q1));
-    for (int col = 0; col < d; ++col)
-      for (int base = 0; base < d; ++base) {
-        if (base & (ba | bb)) continue;
-        const int idx[4] = {base, base | bb, base | ba, base | ba | bb};
-        cd in[4], out[4];
-        for (int r = 0; r < 4; ++r) in[r] = (*U)[idx[r] * d + col];
-        for (int r = 0; r < 4; ++r) {
-          out[r] = 0;
-          for (int cc = 0; cc < 4; ++cc) out[r] += m(4 * r + cc) * in[cc];
-        }
-        for (int r = 0; r < 4; ++r) (*U)[idx[r] * d + col] = out[r];
+    const int ba = 1 << loc(op.q0), bb = 1 << loc(op.q1);
+    const Kind2 kind = classify2(op.m);
+    double out[4][2 * 64];
+    for (int base = 0; base < d; ++base) {
+      if (base & (ba | bb)) continue;
+      double* in[4] = {row(base), row(base | bb), row(base | ba), row(base | ba | bb)};
+      if (kind == K2_CNOT || kind == K2_SWAP) {
+        std::swap_ranges(in[2], in[2] + 2 * d, kind == K2_CNOT ? in[3] : in[1]);
+        continue;
       }
+      if (kind == K2_CZ) {
+        for (int i = 0; i < 2 * d; ++i) in[3][i] = -in[3][i];
+        continue;
+      }
+      for (int r = 0; r < 4; ++r) {
+        std::fill(out[r], out[r] + 2 * d, 0.0);
+        for (int k = 0; k < 4; ++k) {
+          const double re = op.m[2 * (4 * r + k)], im = op.m[2 * (4 * r + k) + 1];
+          if (re == 0.0 && im == 0.0) continue;
+          const double* v = in[k];
+          for (int i = 0; i < 2 * d; i += 2) {
+            out[r][i] += re * v[i] - im * v[i + 1];
+            out[r][i + 1] += re * v[i + 1] + im * v[i];
+          }
+        }
+      }
+      for (int r = 0; r < 4; ++r) std::copy(out[r], out[r] + 2 * d, in[r]);
+    }
     return;
   }
-  const int tb = 1 << loc(int(op.q0));
+  const int tb = 1 << loc(op.q0);
   int cmask = 0;
   if (op.kind == EV_OP_CONTROLLED)
-    for (uint32_t j = 0; j < op.nctrl; ++j) cmask |= 1 << loc(int(c->ctrl_pool[op.ctrl_off + j]));
-  for (int col = 0; col < d; ++col)
-    for (int i0 = 0; i0 < d; ++i0) {
-      if ((i0 & tb) || (i0 & cmask) != cmask) continue;
-      const int i1 = i0 | tb;
-      const cd a0 = (*U)[i0 * d + col], a1 = (*U)[i1 * d + col];
-      (*U)[i0 * d + col] = m(0) * a0 + m(1) * a1;
-      (*U)[i1 * d + col] = m(2) * a0 + m(3) * a1;
-    }
+    for (uint32_t j = 0; j < op.nctrl; ++j) cmask |= 1 << loc(c->ctrl_pool[op.ctrl_off + j]);
+  for (int i0 = 0; i0 < d; ++i0)
+    if (!(i0 & tb) && (i0 & cmask) == cmask) mix_rows(op.m, row(i0), row(i0 | tb), d);
 }
 
 // Greedy fusion: each block starts at the first pending record and takes
@@ -134,29 +152,31 @@ static void apply_to_unitary(const ev_circuit* c, const ev_op& op, const std::ve
 // touch a qubit of a record skipped before it.
 std::vector<Block> fuse_ops(const ev_circuit* c, uint64_t first, uint64_t last, int n, int k) {
   std::vector<Block> blocks;
-  std::vector<uint64_t> pending;
-  for (uint64_t j = first; j < last; ++j) pending.push_back(j);
-  std::vector<int> q;
+  struct Pending {
+    uint64_t op, qubits;
+  };
+  std::vector<Pending> pending, rest;
+  pending.reserve(last - first);
+  for (uint64_t j = first; j < last; ++j) pending.push_back({j, op_qubits(c, c->ops[j])});
+  const uint64_t everything = n >= 64 ? ~uint64_t(0) : (uint64_t(1) << n) - 1;
   const size_t window = 4096;
   while (!pending.empty()) {
     Block b;
     uint64_t fset = 0, blocked = 0;
-    std::vector<uint64_t> rest;
-    size_t scanned = 0;
+    rest.clear();
     for (size_t i = 0; i < pending.size(); ++i) {
-      const ev_op& op = c->ops[pending[i]];
-      op_qubits(c, op, &q);
-      uint64_t qm = 0;
-      for (int x : q) qm |= uint64_t(1) << x;
-      const bool fits = __builtin_popcountll(fset | qm) <= k && (qm & blocked) == 0;
-      if (fits && scanned < window) {
+      if (blocked == everything || i >= window) {  // nothing more can join
+        rest.insert(rest.end(), pending.begin() + ptrdiff_t(i), pending.end());
+        break;
+      }
+      const uint64_t qm = pending[i].qubits;
+      if (__builtin_popcountll(fset | qm) <= k && (qm & blocked) == 0) {
         fset |= qm;
-        b.ops.push_back(pending[i]);
+        b.ops.push_back(pending[i].op);
       } else {
         blocked |= qm;
         rest.push_back(pending[i]);
       }
-      ++scanned;
     }
     // pad F to exactly k qubits with the lowest unused ones
     for (int x = 0; x < n && __builtin_popcountll(fset) < k; ++x) fset |= uint64_t(1) << x;
