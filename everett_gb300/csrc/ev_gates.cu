@@ -81,6 +81,10 @@ __device__ __forceinline__ void pair_update(V* __restrict__ s, uint64_t i0, uint
   }
 }
 
+__device__ __forceinline__ double neg_if(double v, uint64_t flip) {
+  return __longlong_as_double((long long)(uint64_t(__double_as_longlong(v)) ^ flip));
+}
+
 // pair_update with the complex128 products of both outputs on the integer
 // pipes (ev_softpair.cuh); same results.
 template <int KIND>
@@ -92,10 +96,39 @@ __device__ __forceinline__ void pair_update_soft(double2* __restrict__ s, uint64
     s[i1] = a1;
   } else {
     double2 a0 = s[i0], a1 = s[i1];
+    // a sparse state (every one is until its last qubit has been rotated):
+    // nothing to compute or to write.  Zeros are outside the integer-pipe
+    // domain and took the FP64 pipe: dense gates at 26 qubits while half the
+    // register is still in |0>, 1298 us a gate, 190 now.
+    if (zero_amp(a0) && zero_amp(a1)) return;
     soft_pair<KIND>(a0, a1, f, true);
     s[i0] = a0;
     s[i1] = a1;
   }
+}
+
+// A real matrix whose entries share one magnitude (H): m2 a0 and m3 a1 are
+// m0 a0 and m1 a1 up to sign, so 4 products on the integer pipes serve the 8.
+__device__ __forceinline__ bool one_magnitude(const SoftM1& f) {
+  const uint64_t m = softfp::to_bits(f.m0.x) << 1;
+  return (softfp::to_bits(f.m1.x) << 1) == m && (softfp::to_bits(f.m2.x) << 1) == m &&
+         (softfp::to_bits(f.m3.x) << 1) == m;
+}
+__device__ __forceinline__ void pair_update_hadamard(double2* __restrict__ s, uint64_t i0,
+                                                     uint64_t i1, const SoftM1& f, uint64_t flip0,
+                                                     uint64_t flip1) {
+  double2 a0 = s[i0], a1 = s[i1];
+  const SoftAmp s0 = sunpack(a0), s1 = sunpack(a1);
+  if (sok(s0) & sok(s1)) {
+    const double2 p = srmul(f.u0, s0), q = srmul(f.u1, s1);
+    s[i0] = cadd(p, q);
+    s[i1] = cadd(make_double2(neg_if(p.x, flip0), neg_if(p.y, flip0)),
+                 make_double2(neg_if(q.x, flip1), neg_if(q.y, flip1)));
+    return;
+  }
+  if (zero_amp(a0) && zero_amp(a1)) return;
+  s[i0] = cadd(rmul(f.m0.x, a0), rmul(f.m1.x, a1));
+  s[i1] = cadd(rmul(f.m2.x, a0), rmul(f.m3.x, a1));
 }
 
 // An entry in {1, i, -1, -i} as its power of i (0..3), else -1.
@@ -103,9 +136,6 @@ __device__ __forceinline__ int unit_power(double2 m) {
   if (m.y == 0.0) return m.x == 1.0 ? 0 : (m.x == -1.0 ? 2 : -1);
   if (m.x == 0.0) return m.y == 1.0 ? 1 : (m.y == -1.0 ? 3 : -1);
   return -1;
-}
-__device__ __forceinline__ double neg_if(double v, uint64_t flip) {
-  return __longlong_as_double((long long)(uint64_t(__double_as_longlong(v)) ^ flip));
 }
 // i^p a by moving parts and flipping sign bits: the FMA-form product with a
 // unit entry, whose products with the entry's zero part only add +-0, so
@@ -139,6 +169,18 @@ __global__ void __launch_bounds__(256) k_pair(V* __restrict__ s, uint64_t npairs
       }
     }
     const SoftM1 f = soft_matrix<KIND>(m.m0, m.m1, m.m2, m.m3);
+    if constexpr (KIND == K1_REAL) {
+      if (f.ok && one_magnitude(f)) {
+        const uint64_t sign = uint64_t(1) << 63;
+        const uint64_t flip0 = (softfp::to_bits(f.m0.x) ^ softfp::to_bits(f.m2.x)) & sign;
+        const uint64_t flip1 = (softfp::to_bits(f.m1.x) ^ softfp::to_bits(f.m3.x)) & sign;
+        for (uint64_t i = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < npairs; i += stride) {
+          const uint64_t i0 = insert0(i, k);
+          pair_update_hadamard(s, i0, i0 | bit, f, flip0, flip1);
+        }
+        return;
+      }
+    }
     if (f.ok) {
       for (uint64_t i = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < npairs; i += stride) {
         const uint64_t i0 = insert0(i, k);
@@ -195,6 +237,8 @@ __global__ void __launch_bounds__(256) k_pair_shfl(V* __restrict__ s, uint64_t l
             out = cadd(srmul(u0, s0), srmul(u1, s1));
           else
             out = cadd(scmul(r0, u0, a0, s0), scmul(r1, u1, a1, s1));
+        } else if (zero_amp(a0) && zero_amp(a1)) {
+          continue;  // after the loop's shuffle: the whole warp has taken part
         } else if constexpr (KIND == K1_REAL) {
           out = cadd(rmul(r0.x, a0), rmul(r1.x, a1));
         } else {
@@ -235,7 +279,8 @@ __global__ void __launch_bounds__(256) k_diag(V* __restrict__ s, uint64_t len, i
   const uint64_t stride = uint64_t(gridDim.x) * blockDim.x;
   if constexpr (std::is_same<V, double2>::value) {
     const softfp::Unpacked u0 = softfp::unpack(d0.y), u1 = softfp::unpack(d1.y);
-    if (u0.ok & u1.ok) {  // products on the integer pipes, as ev_softpair.cuh
+    // products on the integer pipes, as ev_softpair.cuh
+    if (u0.ok & u1.ok & finite_bits(d0.x) & finite_bits(d1.x)) {
       for (uint64_t j = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; j < len; j += stride) {
         const bool one = (j >> k) & 1;
         s[j] = soft_diag(one ? d1 : d0, one ? u1 : u0, s[j]);
@@ -376,6 +421,8 @@ __global__ void __launch_bounds__(256)
           acc = cadd(acc, scmul(m.m[4 * r + 3], sm.u[4 * r + 3], a[3], ua[3]));
           s[out[r]] = acc;
         }
+      } else if (zero_amp(a[0]) && zero_amp(a[1]) && zero_amp(a[2]) && zero_amp(a[3])) {
+        continue;  // stays zero: the matrix is finite
       } else {
 #pragma unroll
         for (int r = 0; r < 4; ++r) {
@@ -563,7 +610,8 @@ static void go_apply2(ev_state* s, Kind2 kind, uint64_t a, uint64_t b, const dou
 }
 
 // complex128 dense and diagonal 4x4: the integer-pipe products when every
-// imaginary part the kind multiplies by is in softfp's domain.
+// imaginary part the kind multiplies by is in softfp's domain (and the real
+// parts are finite, so that zero amplitudes stay zero).
 template <>
 void go_apply2<double2>(ev_state* s, Kind2 kind, uint64_t a, uint64_t b, const double m[32],
                         const uint8_t* pred) {
@@ -572,7 +620,7 @@ void go_apply2<double2>(ev_state* s, Kind2 kind, uint64_t a, uint64_t b, const d
     uint32_t ok = 1u;
     for (int e = 0; e < 16; ++e) {
       sm.u[e] = softfp::unpack(m[2 * e + 1]);
-      if (kind == K2_DENSE || e % 5 == 0) ok &= sm.u[e].ok;
+      if (kind == K2_DENSE || e % 5 == 0) ok &= sm.u[e].ok & finite_bits(m[2 * e]);
     }
     if (ok) {
       double2* st = static_cast<double2*>(s->amps);

@@ -34,6 +34,14 @@ __device__ __forceinline__ double2 scmul(double2 m, const softfp::Unpacked& my, 
                       __fma_rn(m.x, a.y, softfp::mul(my, ua.x)));
 }
 
+// Tested as bits: comparisons of doubles run on the FP64 pipe.
+__device__ __forceinline__ bool zero_amp(double2 a) {
+  return ((softfp::to_bits(a.x) | softfp::to_bits(a.y)) << 1) == 0;
+}
+__host__ __device__ inline uint32_t finite_bits(double x) {
+  return uint32_t(((softfp::to_bits(x) >> 52) & 0x7FFu) != 0x7FFu);
+}
+
 // The matrix of a record, unpacked once: the real parts for real matrices,
 // the imaginary parts (the factors of the FMA-form product's plain
 // multiplications) otherwise.  ok is set when every factor the kind uses is
@@ -56,9 +64,13 @@ __device__ __forceinline__ SoftM1 soft_matrix(double2 m0, double2 m1, double2 m2
   f.u1 = softfp::unpack(kReal ? m1.x : m1.y);
   f.u2 = softfp::unpack(kReal ? m2.x : m2.y);
   f.u3 = softfp::unpack(kReal ? m3.x : m3.y);
-  if constexpr (K1 == K1_DIAG) f.ok = f.u0.ok & f.u3.ok;
-  else if constexpr (K1 == K1_PHASE) f.ok = f.u3.ok;
-  else if constexpr (K1 == K1_REAL || K1 == K1_DENSE) f.ok = f.u0.ok & f.u1.ok & f.u2.ok & f.u3.ok;
+  // every entry is finite too, so that a zero amplitude's products are zeros
+  if constexpr (K1 == K1_DIAG) f.ok = f.u0.ok & f.u3.ok & finite_bits(m0.x) & finite_bits(m3.x);
+  else if constexpr (K1 == K1_PHASE) f.ok = f.u3.ok & finite_bits(m3.x);
+  else if constexpr (K1 == K1_REAL) f.ok = f.u0.ok & f.u1.ok & f.u2.ok & f.u3.ok;
+  else if constexpr (K1 == K1_DENSE)
+    f.ok = f.u0.ok & f.u1.ok & f.u2.ok & f.u3.ok & finite_bits(m0.x) & finite_bits(m1.x) &
+           finite_bits(m2.x) & finite_bits(m3.x);
   else f.ok = 0;  // anti-diagonal and identity records stay on the FP64 pipe
   return f;
 }
@@ -69,11 +81,13 @@ __device__ __forceinline__ SoftM1 soft_matrix(double2 m0, double2 m1, double2 m2
 __host__ __device__ inline uint32_t soft_factors(int k1, const double* m, softfp::Unpacked u[4]) {
   const int part = k1 == K1_REAL ? 0 : 1;
   for (int j = 0; j < 4; ++j) u[j] = softfp::unpack(m[2 * j + part]);
+  auto fin = [&](int j) { return finite_bits(m[2 * j]); };
   switch (k1) {
-    case K1_DIAG: return u[0].ok & u[3].ok;
-    case K1_PHASE: return u[3].ok;
+    case K1_DIAG: return u[0].ok & u[3].ok & fin(0) & fin(3);
+    case K1_PHASE: return u[3].ok & fin(3);
     case K1_REAL:
-    case K1_DENSE: return u[0].ok & u[1].ok & u[2].ok & u[3].ok;
+    case K1_DENSE:
+      return u[0].ok & u[1].ok & u[2].ok & u[3].ok & fin(0) & fin(1) & fin(2) & fin(3);
     default: return 0;
   }
 }
@@ -82,6 +96,14 @@ __host__ __device__ inline uint32_t soft_factors(int k1, const double* m, softfp
 // operands are in its domain, else on the FP64 pipe: the same bits.
 __device__ __forceinline__ double sadd(double x, double y, bool soft) {
   return (soft && softfp::add_ok(x, y)) ? softfp::add(x, y) : __dadd_rn(x, y);
+}
+
+// One amplitude times a diagonal entry d (du = d.y unpacked), as cmul(d, a);
+// a zero stays itself.
+__device__ __forceinline__ double2 soft_diag(double2 d, const softfp::Unpacked& du, double2 a) {
+  const SoftAmp s = sunpack(a);
+  if (sok(s)) return scmul(d, du, a, s);
+  return zero_amp(a) ? a : cmul(d, a);
 }
 
 // new0 = m0*a0 + m1*a1, new1 = m2*a0 + m3*a1 for a record of kind K1 (REAL,
@@ -111,6 +133,8 @@ __device__ __forceinline__ void soft_pair(double2& a0, double2& a1, const SoftM1
         n1 = both ? cadd(scmul(f.m2, f.u2, a0, s0), scmul(f.m3, f.u3, a1, s1))
                   : cadd(cmul(f.m2, a0), cmul(f.m3, a1));
       }
+    } else if (zero_amp(a0) && zero_amp(a1)) {
+      return;  // a sparse state's pairs stay zero off the FP64 pipe
     } else if constexpr (K1 == K1_REAL) {
       n0 = cadd(rmul(f.m0.x, a0), rmul(f.m1.x, a1));
       n1 = cadd(rmul(f.m2.x, a0), rmul(f.m3.x, a1));
@@ -121,25 +145,11 @@ __device__ __forceinline__ void soft_pair(double2& a0, double2& a1, const SoftM1
     a0 = n0;
     a1 = n1;
   } else if constexpr (K1 == K1_DIAG) {
-    const SoftAmp s0 = sunpack(a0);
-    const double2 n0 = sok(s0) ? scmul(f.m0, f.u0, a0, s0) : cmul(f.m0, a0);
-    if (both) {
-      const SoftAmp s1 = sunpack(a1);
-      a1 = sok(s1) ? scmul(f.m3, f.u3, a1, s1) : cmul(f.m3, a1);
-    } else {
-      a1 = cmul(f.m3, a1);
-    }
-    a0 = n0;
+    a0 = soft_diag(f.m0, f.u0, a0);
+    a1 = both ? soft_diag(f.m3, f.u3, a1) : cmul(f.m3, a1);
   } else if constexpr (K1 == K1_PHASE) {
-    const SoftAmp s1 = sunpack(a1);
-    a1 = sok(s1) ? scmul(f.m3, f.u3, a1, s1) : cmul(f.m3, a1);
+    a1 = soft_diag(f.m3, f.u3, a1);
   }
-}
-
-// One amplitude times a diagonal entry d (du = d.y unpacked), as cmul(d, a).
-__device__ __forceinline__ double2 soft_diag(double2 d, const softfp::Unpacked& du, double2 a) {
-  const SoftAmp s = sunpack(a);
-  return sok(s) ? scmul(d, du, a, s) : cmul(d, a);
 }
 
 }  // namespace ev
