@@ -266,7 +266,7 @@ __device__ __forceinline__ void pauli_channel(const PauliChannel& ch, double2 (&
 template <bool GATE>
 __global__ void __launch_bounds__(kDmThreads, 3)
     k_dm_1q(double2* __restrict__ rho, int n, int t, U1 u, uint64_t mask,
-            const __grid_constant__ PauliChannel ch, const uint8_t* pred) {
+            const __grid_constant__ PauliChannel ch, bool skip_zeros, const uint8_t* pred) {
   if (dm_skip(pred)) return;
   __shared__ SoftU1 su;
   if (GATE) {
@@ -281,9 +281,10 @@ __global__ void __launch_bounds__(kDmThreads, 3)
     const uint64_t r0 = insert0(b >> (n - 1), t), c0 = insert0(b & (half - 1), t);
     const uint64_t r1 = r0 | bit, c1 = c0 | bit;
     double2 e[4] = {rho[r0 * dim + c0], rho[r0 * dim + c1], rho[r1 * dim + c0], rho[r1 * dim + c1]};
-    // a block of zeros stays one (most of rho until every qubit has been
-    // rotated; a zero operand would take the FP64 pipe)
-    if (is_zero(e[0]) & is_zero(e[1]) & is_zero(e[2]) & is_zero(e[3])) continue;
+    // a block of zeros stays one under a finite matrix (most of rho until
+    // every qubit has been rotated; a zero operand would take the FP64 pipe)
+    if ((!GATE || skip_zeros) && (is_zero(e[0]) & is_zero(e[1]) & is_zero(e[2]) & is_zero(e[3])))
+      continue;
     if (GATE) {
       if ((r0 & mask) == mask) {
         left2_any(u.m, f, e[0], e[2]);
@@ -697,9 +698,11 @@ int dm_unitary_1q(ev_dm* d, uint64_t t, const double m[8], uint64_t mask, const 
   U1 u;
   for (int e = 0; e < 4; ++e) u.m[e] = make_double2(m[2 * e], m[2 * e + 1]);
   const uint64_t half = d->dim() / 2;
+  bool finite = true;
+  for (int e = 0; e < 8; ++e) finite = finite && finite_bits(m[e]);
   *applied = ch != nullptr;
   k_dm_1q<true><<<dm_grid(d, half * half), kDmThreads, 0, d->stream>>>(
-      d->rho, int(d->n), int(t), u, mask, ch ? *ch : PauliChannel{}, pred);
+      d->rho, int(d->n), int(t), u, mask, ch ? *ch : PauliChannel{}, finite, pred);
   EV_CUDA(cudaGetLastError());
   return EV_OK;
 }
@@ -728,7 +731,7 @@ int dm_channel(ev_dm* d, const ev_channel& ch, const PauliChannel* pauli, uint64
   const uint64_t half = d->dim() / 2;
   if (pauli != nullptr) {
     k_dm_1q<false><<<dm_grid(d, half * half), kDmThreads, 0, d->stream>>>(
-        d->rho, int(d->n), int(t), U1{}, 0, *pauli, pred);
+        d->rho, int(d->n), int(t), U1{}, 0, *pauli, true, pred);
     EV_CUDA(cudaGetLastError());
     return EV_OK;
   }

@@ -129,6 +129,19 @@ def test_pauli_channels_bit_exact(gpu, name):
         assert np.array_equal(got, want), name
 
 
+@pytest.mark.parametrize("entry", [np.inf, np.nan])
+def test_non_finite_gate_reaches_zero_blocks(gpu, entry):
+    """Blocks of zeros are left alone under finite matrices only: an infinite
+    or NaN entry times zero is NaN."""
+    for noise in ("ideal", "depolarizing"):
+        c = Circuit(3)
+        c.h(0).gate1(Gate1(entry, 0.3j, 0.4, 0.5), 1)
+        want, _ = O.dm_run(c, NOISES[noise].ev_struct())
+        got = DensityMatrixBackend.run_with_noise(c, NOISES[noise]).density_matrix().data()
+        assert np.array_equal(np.isnan(got.real), np.isnan(want.real)), noise
+        assert np.array_equal(np.isnan(got.imag), np.isnan(want.imag)), noise
+
+
 def test_observables_match_oracle(gpu):
     n = 5
     c = mixed_circuit(n, 77)
