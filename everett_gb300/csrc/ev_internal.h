@@ -233,4 +233,25 @@ int resident_blocks() {
   return per_sm;
 }
 
+// Launches a kernel; early: its blocks may start while the stream's previous
+// kernel still runs (programmatic dependent launch), provided that kernel has
+// allowed it (griddepcontrol.launch_dependents) and this one waits
+// (griddepcontrol.wait) before it touches the state.  The next kernel's
+// staging then overlaps this one's tail.
+template <typename... P, typename... A>
+cudaError_t launch_kernel(void (*kernel)(P...), unsigned grid, unsigned block, size_t smem,
+                          cudaStream_t stream, bool early, A... args) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(block);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = early ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+
 }  // namespace ev

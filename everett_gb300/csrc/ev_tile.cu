@@ -219,24 +219,15 @@ static int launch_tile_as(ev_state* s, uint64_t ntiles, size_t smem, const TileP
   ProfScope prof(s, P_TILE, 2.0 * double(s->len()) * double(sizeof(V)));
   s->launches += 1;
   int* derr = reinterpret_cast<int*>(s->scratch.counter + 1);
-  cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3(unsigned(grid));
-  cfg.blockDim = dim3(NT);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = s->stream;
-  cudaLaunchAttribute attr{};
-  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr.val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = &attr;
   // Early launch only where the next pass's blocks find SMs of their own:
   // with more blocks than that they land beside running ones, unevenly, and
   // a pass lasts as long as its fullest SM (complex128, ms per depth-20
   // circuit, early launch on / off: 14 qubits, 64 blocks, 0.61 / 0.64; 15
   // qubits, 128 blocks, 0.85 / 0.68; 20 qubits, 304 blocks of 256 threads,
   // 8.50 / 7.20).
-  cfg.numAttrs = 2 * grid <= uint64_t(s->num_sms) ? 1 : 0;
-  EV_CUDA(cudaLaunchKernelEx(&cfg, k_tile<V, BULK, NT, MINB, STAGES>, static_cast<V*>(s->amps), ntiles,
-                             plan, dops, nops, derr));
+  EV_CUDA(launch_kernel(k_tile<V, BULK, NT, MINB, STAGES>, unsigned(grid), unsigned(NT), smem,
+                        s->stream, 2 * grid <= uint64_t(s->num_sms), static_cast<V*>(s->amps),
+                        ntiles, plan, dops, nops, derr));
   return EV_OK;
 }
 
