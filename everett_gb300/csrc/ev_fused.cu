@@ -435,6 +435,80 @@ struct TcShape {
 
 constexpr uint32_t kWaitLimit = 1u << 24;
 
+// How a pass reaches its amplitudes.  A thread moves its row's values four f
+// at a time; with rows over the lowest qubits a warp's accesses of one f fill
+// whole 32-byte sectors, but when F holds qubit 0 or 1 each touches part of
+// them (F = {0..4}, complex64: 8 of every 256 bytes an access).  Then
+//   LOW_QUADS  F holds qubits 0 and 1: the four values are 32 contiguous
+//              bytes, one access
+//   LOW_PAIRS  F holds qubit 0: two accesses of 16 bytes, adjacent lanes
+//              (rows differing in qubit 1) fill the sector
+//   LOW_CROSS  F holds qubits 1 and 2 but not 0: the 32 bytes of two f and
+//              two adjacent rows are moved as 16 bytes by each of the two
+//              lanes, which exchange halves (with qubit 1 alone the exchange
+//              costs more than it gains: {1, 10..13} 767 without, 872 with)
+// 28 qubits, TF32, us a pass before / after: F = {0..4} 1868 / 1002, {1..5}
+// 1342 / 1016, {0, 1, 20, 21, 22} 947 / 688, {0, 10..13} 723 / 699; sets
+// above qubit 4 670-760.
+enum LowAccess : int { LOW_NONE = 0, LOW_PAIRS = 1, LOW_QUADS = 2, LOW_CROSS = 3 };
+__device__ __forceinline__ int low_access(const FusedDesc& d) {
+  if (d.ftab[1] == 1) return d.ftab[2] == 2 ? LOW_QUADS : LOW_PAIRS;
+  return d.ftab[1] == 2 && d.ftab[2] == 4 ? LOW_CROSS : LOW_NONE;
+}
+__device__ __forceinline__ float2 shfl_pair(float2 v) {
+  return make_float2(__shfl_xor_sync(0xFFFFFFFFu, v.x, 1), __shfl_xor_sync(0xFFFFFFFFu, v.y, 1));
+}
+
+// x[i] = the amplitude of f = f0 + i of the row at rbase (f0 a multiple of 4).
+__device__ __forceinline__ void load_four(const float2* s, uint64_t rbase, const uint64_t* ftab,
+                                          int f0, int low, bool odd, float2 (&x)[4]) {
+  if (low == LOW_NONE) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) x[i] = __ldcs(s + (rbase | ftab[f0 + i]));
+  } else if (low == LOW_QUADS) {
+    asm volatile("ld.global.cs.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                 : "=f"(x[0].x), "=f"(x[0].y), "=f"(x[1].x), "=f"(x[1].y), "=f"(x[2].x),
+                   "=f"(x[2].y), "=f"(x[3].x), "=f"(x[3].y)
+                 : "l"(s + (rbase | ftab[f0])));
+  } else {
+#pragma unroll
+    for (int i = 0; i < 4; i += 2) {
+      const uint64_t at = low == LOW_PAIRS ? rbase | ftab[f0 + i]
+                                           : (rbase & ~uint64_t(1)) | ftab[f0 + i] | (odd ? 2u : 0u);
+      const float4 v = __ldcs(reinterpret_cast<const float4*>(s + at));
+      x[i] = make_float2(v.x, v.y);
+      x[i + 1] = make_float2(v.z, v.w);
+      if (low == LOW_CROSS) {
+        const float2 got = shfl_pair(odd ? x[i] : x[i + 1]);
+        (odd ? x[i] : x[i + 1]) = got;
+      }
+    }
+  }
+}
+__device__ __forceinline__ void store_four(float2* s, uint64_t rbase, const uint64_t* ftab, int f0,
+                                           int low, bool odd, float2 (&x)[4]) {
+  if (low == LOW_NONE) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) __stcs(s + (rbase | ftab[f0 + i]), x[i]);
+  } else if (low == LOW_QUADS) {
+    asm volatile("st.global.cs.v8.f32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(s + (rbase | ftab[f0])),
+                 "f"(x[0].x), "f"(x[0].y), "f"(x[1].x), "f"(x[1].y), "f"(x[2].x), "f"(x[2].y),
+                 "f"(x[3].x), "f"(x[3].y)
+                 : "memory");
+  } else {
+#pragma unroll
+    for (int i = 0; i < 4; i += 2) {
+      const uint64_t at = low == LOW_PAIRS ? rbase | ftab[f0 + i]
+                                           : (rbase & ~uint64_t(1)) | ftab[f0 + i] | (odd ? 2u : 0u);
+      if (low == LOW_CROSS) {
+        const float2 got = shfl_pair(odd ? x[i] : x[i + 1]);
+        (odd ? x[i] : x[i + 1]) = got;
+      }
+      __stcs(reinterpret_cast<float4*>(s + at), make_float4(x[i].x, x[i].y, x[i + 1].x, x[i + 1].y));
+    }
+  }
+}
+
 constexpr int kTcThreads = 256;  // 8 warps: warps w and w+4 share TMEM lane quarter w
 
 template <int KB, int VAR>
@@ -505,15 +579,18 @@ __global__ void __launch_bounds__(kTcThreads, TcShape<KB, VAR>::TC_CTAS)
   const uint32_t rsw = uint32_t((row >> 3) * 1024 + (row & 7) * 128);
   const uint32_t rx = uint32_t(row & 7);
   const uint64_t roff = d.rtab[row];
+  const int low = low_access(d);
+  const bool odd = (tid & 1) != 0;
   const uint32_t lane_tmem = tmem + (uint32_t(quarter * 32) << 16);
-  // L2 prefetch of the rows two steps ahead: contiguous runs of 2^lowbits
+  // L2 prefetch of the next step's rows (28 qubits: 798 us a pass on average,
+  // 815 two steps ahead, 917 without): contiguous runs of 2^lowbits
   // amplitudes, one bulk prefetch per run from warp 1
   const int nruns = 1 << (d.k + 7 - d.lowbits);
   const uint32_t run_bytes = 8u << d.lowbits;
   asm volatile("griddepcontrol.wait;" ::: "memory");  // the previous pass's rows are written
   for (uint64_t step = blockIdx.x; step < d.nsteps && ok; step += gridDim.x) {
-    if (warp == 1 && (tid & 31) < nruns && step + 2 * uint64_t(gridDim.x) < d.nsteps) {
-      const uint64_t b2 = step_base(d, step + 2 * uint64_t(gridDim.x));
+    if (warp == 1 && (tid & 31) < nruns && step + uint64_t(gridDim.x) < d.nsteps) {
+      const uint64_t b2 = step_base(d, step + uint64_t(gridDim.x));
       asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(s + (b2 | d.hitab[tid & 31])),
                    "r"(run_bytes)
                    : "memory");
@@ -523,8 +600,7 @@ __global__ void __launch_bounds__(kTcThreads, TcShape<KB, VAR>::TC_CTAS)
 #pragma unroll
     for (int gi = 0; gi < GPT; ++gi) {
       const int g = half + 2 * gi;
-#pragma unroll
-      for (int i = 0; i < 4; ++i) x[gi][i] = __ldcs(s + (rbase | d.ftab[4 * g + i]));
+      load_four(s, rbase, d.ftab, 4 * g, low, odd, x[gi]);
     }
 #pragma unroll
     for (int gi = 0; gi < GPT; ++gi) {
@@ -604,27 +680,18 @@ __global__ void __launch_bounds__(kTcThreads, TcShape<KB, VAR>::TC_CTAS)
     }
     phase ^= 1;
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    const bool pair_store = d.ftab[1] == 1;  // f bit 0 is qubit 0: outputs a, a+1 adjacent
 #pragma unroll
     for (int c0 = half * (K / 2); c0 < (half + 1) * (K / 2); c0 += 16) {
       uint32_t w[16];
       tmem_ld16(lane_tmem + uint32_t(c0), w);
       asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-      if (pair_store) {
 #pragma unroll
-        for (int j = 0; j < 8; j += 2) {
-          const int a = c0 / 2 + j;
-          __stcs(reinterpret_cast<float4*>(s + (rbase | d.ftab[a])),
-                 make_float4(__uint_as_float(w[2 * j]), __uint_as_float(w[2 * j + 1]),
-                             __uint_as_float(w[2 * j + 2]), __uint_as_float(w[2 * j + 3])));
-        }
-      } else {
+      for (int j = 0; j < 8; j += 4) {
+        float2 y[4];
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          const int a = c0 / 2 + j;
-          __stcs(s + (rbase | d.ftab[a]),
-                 make_float2(__uint_as_float(w[2 * j]), __uint_as_float(w[2 * j + 1])));
-        }
+        for (int i = 0; i < 4; ++i)
+          y[i] = make_float2(__uint_as_float(w[2 * (j + i)]), __uint_as_float(w[2 * (j + i) + 1]));
+        store_four(s, rbase, d.ftab, c0 / 2 + j, low, odd, y);
       }
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -1027,8 +1094,27 @@ __device__ __forceinline__ void oz_load(const double2* p, uint64_t (&v)[2]) {
   v[0] = uint64_t(__double_as_longlong(a.x));
   v[1] = uint64_t(__double_as_longlong(a.y));
 }
+// The bits of the amplitudes f0..f0+3 of the row at rbase.  PAIRS: F holds
+// qubit 0, so two of them are 32 contiguous bytes, one access that fills a
+// sector (26 qubits, F = {0..4}: 838 us a pass with 16-byte accesses,
+// 685 with 32; compiled apart, since both in one kernel cost the other sets
+// 80 us).
+template <bool PAIRS>
+__device__ __forceinline__ void oz_load_four(const double2* s, uint64_t rbase, const uint64_t* ftab,
+                                             int f0, uint64_t (&v)[4][2]) {
+  if constexpr (PAIRS) {
+#pragma unroll
+    for (int i = 0; i < 4; i += 2)
+      asm volatile("ld.global.cs.v4.b64 {%0,%1,%2,%3}, [%4];"
+                   : "=l"(v[i][0]), "=l"(v[i][1]), "=l"(v[i + 1][0]), "=l"(v[i + 1][1])
+                   : "l"(s + (rbase | ftab[f0 + i])));
+  } else {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) oz_load(s + (rbase | ftab[f0 + i]), v[i]);
+  }
+}
 
-template <int ND>
+template <int ND, bool PAIRS>
 __global__ void __launch_bounds__(kOzThreads, 1)
     k_fused_oz(double2* __restrict__ s, const FusedDesc* __restrict__ gd,
                const unsigned char* __restrict__ bmat, int* __restrict__ err) {
@@ -1151,8 +1237,7 @@ __global__ void __launch_bounds__(kOzThreads, 1)
     const uint64_t rb = sb | proff;
 #pragma unroll
     for (int gi = 0; gi < 2; ++gi)
-#pragma unroll
-      for (int i = 0; i < 4; ++i) oz_load(s + (rb | d.ftab[4 * (pq + 4 * gi) + i]), b[gi][i]);
+      oz_load_four<PAIRS>(s, rb, d.ftab, 4 * (pq + 4 * gi), b[gi]);
     em = oz_prepare<ND>(b, err);
   }
   for (int par = 0; step < d.nsteps && ok; step += gridDim.x, par ^= 1) {
@@ -1176,8 +1261,7 @@ __global__ void __launch_bounds__(kOzThreads, 1)
       const uint64_t nb = (((sb | ~cmask) + gbase) & cmask) | proff;
 #pragma unroll
       for (int gi = 0; gi < 2; ++gi)
-#pragma unroll
-        for (int i = 0; i < 4; ++i) oz_load(s + (nb | d.ftab[4 * (pq + 4 * gi) + i]), b[gi][i]);
+        oz_load_four<PAIRS>(s, nb, d.ftab, 4 * (pq + 4 * gi), b[gi]);
     }
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -1231,6 +1315,7 @@ __global__ void __launch_bounds__(kOzThreads, 1)
                                     oz::combine_lo6(__uint_as_float(v[4][c]), __uint_as_float(v[5][c])));
         }
       }
+      [[maybe_unused]] double2 held = make_double2(0.0, 0.0);
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
         const int n = half * 32 + (part & 1) * 16 + c0 + 2 * j;
@@ -1243,7 +1328,15 @@ __global__ void __launch_bounds__(kOzThreads, 1)
         const int p_im = rem + fexp[n + 1] - oz::Fmt<ND>::kPow2Bias;
         const double re = oz::scaled_fp64(acc[2 * j], p_re);
         const double im = (j & 1) ? oz::scaled_fp64(acc[2 * j + 1], p_im) : oz::scaled(acc[2 * j + 1], p_im);
-        __stcs(s + (rbase | d.ftab[n >> 1]), make_double2(re, im));
+        if constexpr (!PAIRS) {
+          __stcs(s + (rbase | d.ftab[n >> 1]), make_double2(re, im));
+        } else if (j & 1) {  // with its neighbour f - 1
+          asm volatile("st.global.cs.v4.f64 [%0], {%1,%2,%3,%4};" ::"l"(s + (rbase | d.ftab[(n >> 1) - 1])),
+                       "d"(held.x), "d"(held.y), "d"(re), "d"(im)
+                       : "memory");
+        } else {
+          held = make_double2(re, im);
+        }
       }
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -1393,18 +1486,18 @@ static void build_bmat_oz(const Block& b, std::vector<unsigned char>* out) {
 // instead of 15.5 (complex128).
 static bool early_pass(const ev_state* s, uint64_t grid) { return 2 * grid <= uint64_t(s->num_sms); }
 
-template <int ND>
+template <int ND, bool PAIRS>
 static int launch_oz(ev_state* s, const FusedDesc* dd, const unsigned char* db, uint64_t nsteps,
                      int* derr) {
-  EV_TRY(prepare_smem_kernel(reinterpret_cast<const void*>(k_fused_oz<ND>)));
+  EV_TRY(prepare_smem_kernel(reinterpret_cast<const void*>(k_fused_oz<ND, PAIRS>)));
   uint64_t grid = uint64_t(s->num_sms);  // one CTA per SM (shared memory and TMEM)
   if (grid > nsteps) grid = nsteps;
   s->tc_ctas_per_sm = 1;
   if (debug_enabled())
     fprintf(stderr, "[ev] k_fused_oz<%d> smem %d per CTA, grid %llu\n", ND, OzShape<ND>::SMEM,
             (unsigned long long)grid);
-  EV_CUDA(launch_kernel(k_fused_oz<ND>, unsigned(grid), kOzThreads, OzShape<ND>::SMEM, s->stream,
-                        early_pass(s, grid), static_cast<double2*>(s->amps), dd, db, derr));
+  EV_CUDA(launch_kernel(k_fused_oz<ND, PAIRS>, unsigned(grid), kOzThreads, OzShape<ND>::SMEM,
+                        s->stream, early_pass(s, grid), static_cast<double2*>(s->amps), dd, db, derr));
   return EV_OK;
 }
 
@@ -1551,6 +1644,7 @@ static int plan_fused(ev_state* s, const ev_circuit* c, uint64_t first, uint64_t
     st.k = int(b.F.size());
     st.variant = variant;
     st.tma = use_tma ? 1 : 0;
+    st.low = b.F[0] == 0 ? 1 : 0;
     st.count = d.nsteps;
     out->push_back(st);
   }
@@ -1565,8 +1659,12 @@ int launch_fused_step(ev_state* s, const SegStep& st, const unsigned char* dblob
   s->launches += 1;
   const uint64_t nsteps = st.count;
   const bool tma = st.tma != 0;
-  if (st.variant == EV_FUSED_OZAKI) return launch_oz<7>(s, dd, dm, nsteps, derr);
-  if (st.variant == EV_FUSED_OZAKI6) return launch_oz<6>(s, dd, dm, nsteps, derr);
+  if (st.variant == EV_FUSED_OZAKI)
+    return st.low ? launch_oz<7, true>(s, dd, dm, nsteps, derr)
+                  : launch_oz<7, false>(s, dd, dm, nsteps, derr);
+  if (st.variant == EV_FUSED_OZAKI6)
+    return st.low ? launch_oz<6, true>(s, dd, dm, nsteps, derr)
+                  : launch_oz<6, false>(s, dd, dm, nsteps, derr);
   if (st.variant == EV_FUSED_TF32X3)
     return tma ? launch_tma<5, EV_FUSED_TF32X3, 3>(s, dd, dm, nsteps, derr)
                : launch_tc<5, EV_FUSED_TF32X3>(s, dd, dm, nsteps, derr);

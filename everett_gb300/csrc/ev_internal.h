@@ -166,6 +166,7 @@ struct SegStep {
   int k = 0;            // fused: qubits per unitary
   int variant = 0;      // fused: EV_FUSED_*
   int tma = 0;          // fused: TMA-staged pipeline
+  int low = 0;          // fused: the unitary's qubits include qubit 0
   uint64_t count = 0;   // tile: tiles; fused: 128-row steps
 };
 

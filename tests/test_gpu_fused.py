@@ -199,3 +199,26 @@ def test_ozaki_rejects_complex64_and_complex64_variants_reject_complex128(gpu):
             CudaStateVectorBackend.run(c, dtype="complex64", mode="fused", variant=v)
     with pytest.raises(E.EverettError):
         CudaStateVectorBackend.run(c, dtype="complex128", mode="fused", variant="bf16x3")
+
+
+@pytest.mark.parametrize("F", [(0, 1, 2, 3, 4), (0, 1, 5, 8, 12), (0, 2, 3, 4, 5), (0, 2, 7, 9, 11),
+                               (1, 2, 3, 4, 5), (1, 2, 8, 10, 12), (1, 3, 4, 5, 6), (1, 4, 7, 9, 12),
+                               (2, 3, 4, 5, 6), (8, 9, 10, 11, 12)])
+@pytest.mark.parametrize("variant", ["tf32x3", "bf16x3", "ozaki", "ozaki6"])
+def test_low_qubit_access_forms(gpu, F, variant):
+    """One dense block on qubits F after a layer over the register: the ways
+    a pass reaches its amplitudes when F holds qubits 0, 1 or 2 (32-byte
+    accesses of four or two values, 16-byte pairs, halves exchanged between
+    lanes) against the oracle: 1e-12 in complex128, 1e-5 in complex64."""
+    n = 13
+    rng = np.random.default_rng(sum(F))
+    c = workloads.random_layers(n, 1, seed=sum(F))
+    for _ in range(2):
+        for q in F:
+            c.ry(q, rng.uniform(0, 6)).rz(q, rng.uniform(0, 6))
+        for a, b in zip(F, F[1:]):
+            c.cnot(a, b)
+    want, _, _ = O.run_seeded(c, 0)
+    dtype = "complex128" if variant.startswith("ozaki") else "complex64"
+    got = CudaStateVectorBackend.run(c, dtype=dtype, mode="fused", variant=variant).state().amplitudes()
+    assert np.max(np.abs(got - want)) < (1e-12 if dtype == "complex128" else 1e-5)
