@@ -286,9 +286,12 @@ __global__ void __launch_bounds__(NT, STAGES ? 512 / NT : NT == 256 ? 3 : 2) k_b
   V* tile = reinterpret_cast<V*>(sm);
   uint64_t* offs = reinterpret_cast<uint64_t*>(sm + (sizeof(V) << kmax));
   double* red = reinterpret_cast<double*>(offs + (size_t(1) << (kmax > 4 ? kmax - 4 : 0)));
-  // staged records and their matrices: [window records][window slots]
-  const size_t stage_at = (reinterpret_cast<size_t>(red + 2 * blockDim.x) + 15) & ~size_t(15);
-  BatchOp* srec = reinterpret_cast<BatchOp*>(stage_at);
+  // staged records and their matrices: [window records][window slots], at an
+  // offset from sm (an address rounded up as an integer would make them
+  // generic pointers: 64-bit addressing and generic loads in every record)
+  const uint32_t red_end = (uint32_t(sizeof(V)) << kmax) +
+                           (8u << (kmax > 4 ? kmax - 4 : 0)) + 16u * blockDim.x;
+  BatchOp* srec = reinterpret_cast<BatchOp*>(sm + ((red_end + 15u) & ~15u));
   double* smat = reinterpret_cast<double*>(srec + a.window);
   constexpr uint32_t kSlot = mat_slot_doubles<V>();
   __shared__ uint32_t s_matoff[kMaxWindow];
