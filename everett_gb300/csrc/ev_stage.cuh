@@ -135,15 +135,22 @@ __device__ __forceinline__ void reg_diag(float2 (&a)[R], float2 d0, float2 d1) {
     own_case<POS>();
   }
 }
-// Register r times e[2 * bit Y + bit X].
+// Register r times entry 2 * bit Y + bit X of the diagonal of the 4x4 mm.
 template <int X, int Y, int R>
-__device__ __forceinline__ void reg_diag2(float2 (&a)[R], const float2 (&e)[4]) {
+__device__ __forceinline__ void reg_diag2(float2 (&a)[R], const double* mm) {
   if constexpr ((1 << Y) < R) {
     own_case<8 * Y + X>();
+    const float2 e[4] = {ldm<float2>(mm, 0), ldm<float2>(mm, 5), ldm<float2>(mm, 10),
+                         ldm<float2>(mm, 15)};
 #pragma unroll
     for (int r = 0; r < R; ++r) mul_to(e[2 * ((r >> Y) & 1) + ((r >> X) & 1)], a[r]);
     own_case<8 * Y + X>();
   }
+}
+// The same with p0 at register bit POS and p1's bit, b1, among the threads.
+template <int POS, int R>
+__device__ __forceinline__ void reg_diag2_half(float2 (&a)[R], const double* mm, uint32_t b1) {
+  reg_diag<POS>(a, ldm<float2>(mm, int(5u * b1)), ldm<float2>(mm, int(10u + 5u * b1)));
 }
 // Exchanges the registers that differ in bit T and have the control bit C.
 template <int C, int T, int R, typename F>
@@ -196,10 +203,9 @@ enum StageCode : uint8_t {
   SC_CNOT_REG = 70,       // + 4 * target bit + control bit
   SC_SWAP = 86,           // + pair
   SC_DENSE2 = 92,
-  SC_DIAG2 = 93,          // + pair: entry by both register bits
-  SC_DIAG2_FIRST = 99,    // + bit of p0, p1 among the threads
-  SC_DIAG2_SECOND = 103,  // + bit of p1, p0 among the threads
-  SC_DIAG2_THREAD = 107
+  SC_DIAG2 = 93,          // + pair: entry by both register bits, p0 the higher
+  SC_DIAG2_HALF = 99,     // + bit of p0, p1 among the threads
+  SC_DIAG2_THREAD = 103   // both among the threads
 };
 // Index 0..5 of an unordered pair of register bits x < y.
 __host__ __device__ __forceinline__ int bit_pair(int x, int y) { return x + (y * (y - 1)) / 2; }
@@ -318,33 +324,15 @@ __device__ __forceinline__ void stage_record(float2 (&a)[R], uint32_t l0, const 
       }
       break;
     }
-    default: {
-      if (code >= SC_DIAG2 && code <= SC_DIAG2_THREAD) {
-        // entry 2 * bit(p0) + bit(p1) of the diagonal
-        const uint32_t b0 = (l0 >> op.p0) & 1u, b1 = (l0 >> op.p1) & 1u;
-        const bool up = (op.ins & 15u) > ((op.ins >> 4) & 15u);  // p0 at the higher register bit
-        const float2 e[4] = {m0, ldm<float2>(mm, up ? 5 : 10), ldm<float2>(mm, up ? 10 : 5),
-                             ldm<float2>(mm, 15)};
-        switch (code) {
-          EV_PAIRS(SC_DIAG2, reg_diag2, e)
-          case SC_DIAG2_THREAD: {
-            const float2 d = ldm<float2>(mm, int(5u * (2u * b0 + b1)));
-            reg_subset<0>(a, [=](float2& x) { mul_to(d, x); });
-            break;
-          }
-          default: {
-            const bool first = code < SC_DIAG2_SECOND;
-            const float2 lo = ldm<float2>(mm, int(first ? 5u * b1 : 10u * b0));
-            const float2 hi = ldm<float2>(mm, int(first ? 10u + 5u * b1 : 10u * b0 + 5u));
-            switch (code - (first ? SC_DIAG2_FIRST : SC_DIAG2_SECOND)) {
-              EV_BITS(0, reg_diag, lo, hi)
-            }
-            break;
-          }
-        }
-      }
-      break;  // SC_NONE
+    EV_PAIRS(SC_DIAG2, reg_diag2, mm)
+    EV_BITS(SC_DIAG2_HALF, reg_diag2_half, mm, (l0 >> op.p1) & 1u)
+    case SC_DIAG2_THREAD: {
+      const uint32_t b0 = (l0 >> op.p0) & 1u, b1 = (l0 >> op.p1) & 1u;
+      const float2 d = ldm<float2>(mm, int(5u * (2u * b0 + b1)));
+      reg_subset<0>(a, [=](float2& x) { mul_to(d, x); });
+      break;
     }
+    default: break;  // SC_NONE
   }
 #undef EV_BITS
 #undef EV_PAIRS
@@ -444,7 +432,7 @@ inline uint8_t stage_code(const TileOp& o, int b0, int b1, uint32_t rmask) {
     case T_SWAP: return uint8_t(SC_SWAP + pair);
     case T_DIAG2:
       if (b0 < 15 && b1 < 15) return uint8_t(SC_DIAG2 + pair);
-      return uint8_t(b0 < 15 ? SC_DIAG2_FIRST + b0 : b1 < 15 ? SC_DIAG2_SECOND + b1 : SC_DIAG2_THREAD);
+      return uint8_t(b0 < 15 ? SC_DIAG2_HALF + b0 : SC_DIAG2_THREAD);
     default: return SC_DENSE2;
   }
 }
@@ -499,7 +487,18 @@ inline void mark_stages(TileOp* ops, size_t nops, int k, size_t maxrun) {
           if (pos[b] == p) return b;
         return 15;
       };
-      const int b0 = bit_of(o.p0), b1 = o.kind == T_1Q ? 15 : bit_of(o.p1);
+      int b0 = bit_of(o.p0), b1 = o.kind == T_1Q ? 15 : bit_of(o.p1);
+      // a diagonal takes its operands in either order: p0 at the higher
+      // register bit, or the one that has a register bit
+      if (o.kind == T_DIAG2 && (b0 == 15 || (b1 != 15 && b1 > b0)) && b1 != 15) {
+        std::swap(b0, b1);
+        std::swap(o.p0, o.p1);
+        float f[32];  // entries 5 and 10 trade places
+        std::memcpy(f, o.m, sizeof(f));
+        std::swap(f[10], f[20]);
+        std::swap(f[11], f[21]);
+        std::memcpy(o.m, f, sizeof(f));
+      }
       uint32_t rmask = 0;
       if (o.kind == T_1Q) {
         for (int b = 0; b < np; ++b)
