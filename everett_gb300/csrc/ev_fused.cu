@@ -973,18 +973,29 @@ __global__ void __launch_bounds__(kTmaThreads)
 // threads of a row (lanes l, l + 8, l + 16, l + 24) take the row's largest
 // exponent with two shuffles, and the eight lanes of a store phase hold
 // eight different rows (their 16-byte chunks land in eight bank groups).
-// Recombination: thread t reads TMEM lane t mod 128 (its row), output
-// columns 16 (t / 128) .. + 15.
+// Recombination: thread t reads TMEM lane t mod 128 (its row), columns
+// 8 (t / 128) .. + 7 of each output half.
 //
-// A step s: the workers write the A slices from the prepared digits of s,
-// start loading the rows of s + 1, meet at a barrier (wbar: an mbarrier, so
-// that the wait is bounded) and signal the MMA warp (abar); its lane 0 issues the MMAs of output half 0 (committed to
-// bar[0]) and half 1 (bar[1]) -- issue blocks at about the tensor core's
-// pace, hence a warp of its own; meanwhile the workers prepare s + 1
-// (largest exponent, fixed-point values), then recombine s once its half is
-// done.  A worker's arrival at the barrier of s + 1 also means its TMEM reads
-// of s are complete.  Every wait is bounded; on timeout the kernel records an
-// error, frees TMEM and returns.
+// The MMA warp's lane 0 issues the MMAs of output half 0 (committed to
+// bar[0]) and half 1 (bar[1]); issue blocks at about the tensor core's pace,
+// hence a warp of its own.  The A slices are free once both are done, so a
+// worker's step s runs: recombine half 0 (under the MMAs of half 1); write
+// the A slices of s + 1 from the prepared digits and arrive at abar, which
+// starts half 0 of s + 1; start loading the rows of s + 2; recombine half 1
+// (tbar: read, half 1 of s + 1 may start); prepare s + 2 (largest exponent,
+// fixed-point values).  Every wait is bounded; on timeout the kernel records
+// an error, frees TMEM and returns.
+//
+// What bounds it: the workers' ALU and FP64 conversions (26 qubits: about
+// 8000 clk a step against 4900 for the MMAs and 5700 for its bytes at copy
+// rate).  One pass at 26 qubits, random layers: 660 us with the slices of
+// s + 1 written after all of s was recombined and a range test on each
+// output; 648 in the order above; 522 with one range test a row, so that the
+// conversions of a thread overlap, and fixed-point values formed without
+// branches; 518 with the slices written as shared memory; 492 with every
+// output converted on the FP64 pipe (three in four: 518, half: 550); 479 with
+// three permutes for two digits and byte offsets in place of indices.  Slower:
+// half of the warps recombining while the others prepare (527 and 543).
 
 constexpr int kOzWorkers = 512;                // 16 worker warps
 constexpr int kOzThreads = kOzWorkers + 32;    // and the MMA warp
@@ -1010,12 +1021,15 @@ __device__ __forceinline__ uint32_t hsub2_bits(uint32_t a, uint32_t b) {
   return u;
 }
 
-// FP16 digits (u - 128) of byte k of w0 and of w1, packed [w0's | w1's << 16]:
-// f16 bits 0x6400 | u are 1024 + u, and 1024 + u - 1152 is exact.
-template <int k>
-__device__ __forceinline__ uint32_t oz_byte_digits(uint32_t w0, uint32_t w1) {
-  const uint32_t t = __byte_perm(w0, w1, uint32_t(k | ((k + 4) << 8)));
-  return hsub2_bits((t & 0x00FF00FFu) | 0x64006400u, 0x64806480u);
+// FP16 digits (u - 128) of bytes 2 h and 2 h + 1 of w0 and of w1, packed
+// [w0's | w1's << 16]: f16 bits 0x6400 | u are 1024 + u, and 1024 + u - 1152
+// is exact.  Three byte permutes for two digits, as the ALU bounds a step's
+// workers (a permute, a mask and an or for each: four).
+template <int h>
+__device__ __forceinline__ void oz_byte_digits(uint32_t w0, uint32_t w1, uint32_t& even, uint32_t& odd) {
+  const uint32_t p = __byte_perm(w0, w1, h == 0 ? 0x5140 : 0x7362);  // w0, w1 by turns
+  even = hsub2_bits(__byte_perm(p, 0x64646464u, 0x4140), 0x64806480u);
+  odd = hsub2_bits(__byte_perm(p, 0x64646464u, 0x4342), 0x64806480u);
 }
 
 // The ND FP16 digits of two biased fixed-point values (b = M + kBias),
@@ -1031,19 +1045,12 @@ __device__ __forceinline__ void oz_digits(uint64_t b0, uint64_t b1, uint32_t w[N
   const uint32_t t1 = uint32_t(0x6600 + (int32_t(h1) >> tsh));
   w[0] = hsub2_bits(__byte_perm(t0, t1, 0x5410), 0x66006600u);
   if constexpr (ND == 7) {
-    w[1] = oz_byte_digits<1>(h0, h1);
-    w[2] = oz_byte_digits<0>(h0, h1);
-    w[3] = oz_byte_digits<3>(l0, l1);
-    w[4] = oz_byte_digits<2>(l0, l1);
-    w[5] = oz_byte_digits<1>(l0, l1);
-    w[6] = oz_byte_digits<0>(l0, l1);
+    oz_byte_digits<0>(h0, h1, w[2], w[1]);
   } else {
-    w[1] = oz_byte_digits<0>(h0, h1);
-    w[2] = oz_byte_digits<3>(l0, l1);
-    w[3] = oz_byte_digits<2>(l0, l1);
-    w[4] = oz_byte_digits<1>(l0, l1);
-    w[5] = oz_byte_digits<0>(l0, l1);
+    w[1] = hsub2_bits((__byte_perm(h0, h1, 0x0400) & 0x00FF00FFu) | 0x64006400u, 0x64806480u);
   }
+  oz_byte_digits<1>(l0, l1, w[ND - 3], w[ND - 4]);
+  oz_byte_digits<0>(l0, l1, w[ND - 1], w[ND - 2]);
 }
 
 __device__ __forceinline__ void mma_f16(uint32_t dtmem, uint64_t a, uint64_t b, uint32_t idesc,
@@ -1067,13 +1074,14 @@ __device__ __forceinline__ void tmem_ld8(uint32_t taddr, uint32_t v[8]) {
 // threads: lanes l, l + 8, l + 16, l + 24).
 template <int ND>
 __device__ __forceinline__ int oz_prepare(uint64_t (&v)[2][4][2], int* err) {
-  int em = 0;
+  uint32_t top = 0;
 #pragma unroll
   for (int gi = 0; gi < 2; ++gi)
 #pragma unroll
     for (int i = 0; i < 4; ++i)
 #pragma unroll
-      for (int c = 0; c < 2; ++c) em = max(em, oz::exp_of(uint32_t(v[gi][i][c] >> 32)));
+      for (int c = 0; c < 2; ++c) top = max(top, uint32_t(v[gi][i][c] >> 32) & 0x7FFFFFFFu);
+  int em = oz::exp_of(top);
   em = max(em, __shfl_xor_sync(0xFFFFFFFFu, em, 8));
   em = max(em, __shfl_xor_sync(0xFFFFFFFFu, em, 16));
   if (em == 0x7FF) atomicCAS(err, 0, kFlagNonFinite);  // NaN or infinity in the row
@@ -1083,8 +1091,7 @@ __device__ __forceinline__ int oz_prepare(uint64_t (&v)[2][4][2], int* err) {
     for (int i = 0; i < 4; ++i)
 #pragma unroll
       for (int c = 0; c < 2; ++c)
-        v[gi][i][c] = uint64_t(oz::fixed<ND>(uint32_t(v[gi][i][c] >> 32), uint32_t(v[gi][i][c]), em)) +
-                      oz::Fmt<ND>::kBias;
+        v[gi][i][c] = oz::biased<ND>(uint32_t(v[gi][i][c] >> 32), uint32_t(v[gi][i][c]), em);
   return em;
 }
 
@@ -1094,23 +1101,22 @@ __device__ __forceinline__ void oz_load(const double2* p, uint64_t (&v)[2]) {
   v[0] = uint64_t(__double_as_longlong(a.x));
   v[1] = uint64_t(__double_as_longlong(a.y));
 }
-// The bits of the amplitudes f0..f0+3 of the row at rbase.  PAIRS: F holds
-// qubit 0, so two of them are 32 contiguous bytes, one access that fills a
-// sector (26 qubits, F = {0..4}: 838 us a pass with 16-byte accesses,
-// 685 with 32; compiled apart, since both in one kernel cost the other sets
-// 80 us).
+// The bits of four amplitudes of the row at p, at the byte offsets fofs.
+// PAIRS: F holds qubit 0, so two of them are 32 contiguous bytes, one access
+// that fills a sector (26 qubits, F = {0..4}: 838 us a pass with 16-byte
+// accesses, 685 with 32; compiled apart, since both in one kernel cost the
+// other sets 80 us).
 template <bool PAIRS>
-__device__ __forceinline__ void oz_load_four(const double2* s, uint64_t rbase, const uint64_t* ftab,
-                                             int f0, uint64_t (&v)[4][2]) {
+__device__ __forceinline__ void oz_load_four(const char* p, const uint64_t* fofs, uint64_t (&v)[4][2]) {
   if constexpr (PAIRS) {
 #pragma unroll
     for (int i = 0; i < 4; i += 2)
       asm volatile("ld.global.cs.v4.b64 {%0,%1,%2,%3}, [%4];"
                    : "=l"(v[i][0]), "=l"(v[i][1]), "=l"(v[i + 1][0]), "=l"(v[i + 1][1])
-                   : "l"(s + (rbase | ftab[f0 + i])));
+                   : "l"(p + fofs[i]));
   } else {
 #pragma unroll
-    for (int i = 0; i < 4; ++i) oz_load(s + (rbase | ftab[f0 + i]), v[i]);
+    for (int i = 0; i < 4; ++i) oz_load(reinterpret_cast<const double2*>(p + fofs[i]), v[i]);
   }
 }
 
@@ -1125,13 +1131,15 @@ __global__ void __launch_bounds__(kOzThreads, 1)
   // the next pass may stage its operands now; its workers wait for this one
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   __shared__ __align__(8) uint64_t bar[2];
-  __shared__ __align__(8) uint64_t abar;  // A slices of a step written
-  __shared__ __align__(8) uint64_t wbar;  // all workers past their digit writes
+  __shared__ __align__(8) uint64_t abar;  // a step's A slices written, output half 0 of the one before read
+  __shared__ __align__(8) uint64_t tbar;  // a step's output half 1 read
   __shared__ uint32_t tmem_slot;
-  __shared__ int fexp[K];
+  __shared__ __align__(16) int fexp[K];       // column exponents less kPow2Bias
+  __shared__ __align__(16) uint32_t fhi[K];   // the same in an f64's exponent field
+  __shared__ __align__(16) uint64_t fofs[K / 2];  // byte offset of amplitude f of a row
   __shared__ int rowexp[2][kRows];
-  unsigned char* sm = reinterpret_cast<unsigned char*>(
-      (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  // by an offset, so that the slices are written as shared memory
+  unsigned char* sm = smem_raw + ((1024 - (smem_addr(smem_raw) & 1023)) & 1023);
   unsigned char* a_sl = sm;
   unsigned char* b_sl = sm + ND * Sh::A_SLICE;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -1147,14 +1155,17 @@ __global__ void __launch_bounds__(kOzThreads, 1)
       *reinterpret_cast<uint16_t*>(b_sl + sw128_off(brow, k, ND * K, 2)) = src[e];
     }
     const int* fe = reinterpret_cast<const int*>(bmat + ND * Sh::B_SLICE);
-    for (int n = tid; n < K; n += blockDim.x) fexp[n] = fe[n];
+    for (int n = tid; n < K; n += blockDim.x) {
+      fexp[n] = fe[n] - oz::Fmt<ND>::kPow2Bias;
+      fhi[n] = uint32_t(fexp[n]) << 20;
+    }
+    for (int f = tid; f < K / 2; f += blockDim.x) fofs[f] = gd->ftab[f] * sizeof(double2);
   }
   if (tid == 0) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_addr(&bar[0])));
     asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_addr(&bar[1])));
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_addr(&abar)));
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_addr(&wbar)),
-                 "n"(kOzWorkers));
+    mbar_init(&abar, kOzWorkers / 32);
+    mbar_init(&tbar, kOzWorkers / 32);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 0) {
@@ -1174,15 +1185,21 @@ __global__ void __launch_bounds__(kOzThreads, 1)
       // descriptor start addresses are address >> 4: offsets add directly
       const uint64_t ad = sw128_desc(smem_addr(a_sl)), bd = sw128_desc(smem_addr(b_sl));
       uint32_t aphase = 0;
-      for (uint64_t st = blockIdx.x; st < d.nsteps; st += gridDim.x) {
+      bool done = false;
+      for (uint64_t st = blockIdx.x; st < d.nsteps && !done; st += gridDim.x) {
         if (!mbar_wait(&abar, aphase, kWaitLimit)) {
           atomicExch(err, 1);
           break;
         }
-        aphase ^= 1;
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll 1
         for (int h = 0; h < 2; ++h) {
+          // the previous step's second half has been read
+          if (h == 1 && st != blockIdx.x && !mbar_wait(&tbar, aphase ^ 1, kWaitLimit)) {
+            atomicExch(err, 1);
+            done = true;
+            break;
+          }
+          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll 1
           for (int i = 0; i < ND; ++i) {
             const uint32_t n = uint32_t(32 * (ND - i));
@@ -1200,6 +1217,7 @@ __global__ void __launch_bounds__(kOzThreads, 1)
                   smem_addr(&bar[h]))
               : "memory");
         }
+        aphase ^= 1;
       }
     }
     __syncwarp();
@@ -1207,8 +1225,6 @@ __global__ void __launch_bounds__(kOzThreads, 1)
     return;  // TMEM is freed by warp 0
   }
   asm volatile("griddepcontrol.wait;" ::: "memory");  // the previous pass's rows are written
-  uint32_t phase = 0;
-  bool ok = true;
   // preparation role: the eight lanes of a store phase hold eight different
   // rows, so their 16-byte chunks land in eight different bank groups
   const int prow = 8 * warp + (lane & 7), pq = lane >> 3;
@@ -1216,32 +1232,39 @@ __global__ void __launch_bounds__(kOzThreads, 1)
   const uint32_t prx = uint32_t(prow & 7);
   const uint64_t proff = d.rtab[prow];
   // recombination role
-  const int quarter = warp & 3, part = warp >> 2, half = part >> 1;
-  const int erow = quarter * 32 + lane;
+  const int erow = (warp & 3) * 32 + lane, part = warp >> 2;
   const uint64_t eroff = d.rtab[erow];
-  const uint32_t lane_tmem = tmem + (uint32_t(quarter * 32) << 16);
-  const uint32_t col0 = uint32_t(half * Sh::HALF_COLS + (part & 1) * 16);
+  const uint32_t lane_tmem = tmem + (uint32_t((warp & 3) * 32) << 16);
+  // the columns' range of exponents; a zero column's sums are zero, as a zero
+  // row's are, whatever the exponent
+  int flo = 4096, ftop = -4096;
+  for (int n = lane; n < K; n += 32)
+    if (fexp[n] != -oz::Fmt<ND>::kPow2Bias) {
+      flo = min(flo, fexp[n]);
+      ftop = max(ftop, fexp[n]);
+    }
+  flo = __reduce_min_sync(0xFFFFFFFFu, flo);
+  ftop = __reduce_max_sync(0xFFFFFFFFu, ftop);
 
   uint64_t b[2][4][2];  // the rows' bits, then their biased fixed-point values
   int em = 0;
-  uint64_t step = blockIdx.x;
   // Step bases advance by a masked add: with M the mask of the step-index
   // qubits, base(s + grid) = ((base(s) | ~M) + base(grid)) & M.
   uint64_t cmask = 0;
   for (int q = 0; q < d.ncomp_hi; ++q) cmask |= uint64_t(1) << d.comp_hi[q];
   const uint64_t gbase = step_base(d, gridDim.x);
+  auto advance = [&](uint64_t base) { return ((base | ~cmask) + gbase) & cmask; };
   const int nruns = 1 << (d.k + 7 - d.lowbits);  // the 2^(k+7) amplitudes of a step
   const uint32_t run_bytes = 16u << d.lowbits;
-  uint64_t sb = step_base(d, step);
-  if (step < d.nsteps) {
-    const uint64_t rb = sb | proff;
+
+  auto load = [&](uint64_t base) {
 #pragma unroll
     for (int gi = 0; gi < 2; ++gi)
-      oz_load_four<PAIRS>(s, rb, d.ftab, 4 * (pq + 4 * gi), b[gi]);
-    em = oz_prepare<ND>(b, err);
-  }
-  for (int par = 0; step < d.nsteps && ok; step += gridDim.x, par ^= 1) {
-    // A slices of this step from the prepared digits
+      oz_load_four<PAIRS>(reinterpret_cast<const char*>(s + (base | proff)), fofs + 4 * (pq + 4 * gi), b[gi]);
+  };
+  // the A slices of the step whose prepared digits b and em hold; the warp's
+  // arrival hands them to the MMA warp
+  auto write_slices = [&](int par) {
 #pragma unroll
     for (int gi = 0; gi < 2; ++gi) {
       const int g = pq + 4 * gi;  // reals 8g..8g+7: chunk g of the row's 128-byte line
@@ -1255,52 +1278,29 @@ __global__ void __launch_bounds__(kOzThreads, 1)
             make_uint4(w[0][sl], w[1][sl], w[2][sl], w[3][sl]);
     }
     if (pq == 0) rowexp[par][prow] = em;
-    // the next step's rows, in flight while the MMAs are issued
-    const uint64_t nstep = step + gridDim.x;
-    if (nstep < d.nsteps) {
-      const uint64_t nb = (((sb | ~cmask) + gbase) & cmask) | proff;
-#pragma unroll
-      for (int gi = 0; gi < 2; ++gi)
-        oz_load_four<PAIRS>(s, nb, d.ftab, 4 * (pq + 4 * gi), b[gi]);
-    }
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    // the workers meet (every one arrives, the wait is bounded), then the
-    // MMA warp is told that the A slices of this step are complete
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_addr(&wbar)) : "memory");
-    if (!mbar_wait(&wbar, phase, kWaitLimit)) {
-      ok = false;
-      atomicExch(err, 1);
-      break;
-    }
-    if (tid == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_addr(&abar)) : "memory");
-    // the rows of the step after next into L2 (contiguous runs of 2^lowbits
-    // amplitudes, at most 32 of them), so that next step's loads hit L2
-    if (warp == 1 && lane < nruns && nstep + gridDim.x < d.nsteps) {
-      const uint64_t b2 = (((((sb | ~cmask) + gbase) & cmask) | ~cmask) + gbase) & cmask;
-      asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(s + (b2 | d.hitab[lane])),
-                   "r"(run_bytes)
-                   : "memory");
-    }
-    // prepare the next step while the tensor core works
-    if (nstep < d.nsteps) em = oz_prepare<ND>(b, err);
-    if (!mbar_wait(&bar[half], phase, kWaitLimit)) {
-      ok = false;
-      atomicExch(err, 1);
-      break;
-    }
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    const int rem = rowexp[par][erow];
-    const uint64_t rbase = sb | eroff;
-#pragma unroll
-    for (int c0 = 0; c0 < 16; c0 += 8) {
-      const uint32_t ta = lane_tmem + col0 + uint32_t(c0);
+    __syncwarp();
+    if (lane == 0)
+      asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_addr(&abar)) : "memory");
+  };
+  // this thread's eight columns of one output half
+  auto recombine = [&](int half, char* row, int rem, bool plain) {
+    {
+      const int n0 = part * 8;
+      const uint32_t ta = lane_tmem + uint32_t(half * Sh::HALF_COLS + n0);
       int64_t acc[8];
       {
         uint32_t v[ND][8];
 #pragma unroll
         for (int dg = 0; dg < ND; ++dg) tmem_ld8(ta + uint32_t(32 * dg), v[dg]);
         asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+        if (half == 1) {
+          asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+          __syncwarp();
+          if (lane == 0)
+            asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_addr(&tbar)) : "memory");
+        }
 #pragma unroll
         for (int c = 0; c < 8; ++c) {
           int32_t g3, g2;
@@ -1315,40 +1315,86 @@ __global__ void __launch_bounds__(kOzThreads, 1)
                                     oz::combine_lo6(__uint_as_float(v[4][c]), __uint_as_float(v[5][c])));
         }
       }
+      const int n1 = half * 32 + n0;
+      const uint64_t* fo = fofs + (n1 >> 1);
       [[maybe_unused]] double2 held = make_double2(0.0, 0.0);
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const int n = half * 32 + (part & 1) * 16 + c0 + 2 * j;
-        // three outputs in four converted on the FP64 pipe, which is idle
-        // while the integer pipes recombine, the fourth on the integer pipes:
-        // the same values either way.  30 qubits, ms per run (seven / six
-        // digits): all on the integer pipes 903 / 865, half on FP64 838 /
-        // 800, three quarters 825 / 771, all 832 / 766
-        const int p_re = rem + fexp[n] - oz::Fmt<ND>::kPow2Bias;
-        const int p_im = rem + fexp[n + 1] - oz::Fmt<ND>::kPow2Bias;
-        const double re = oz::scaled_fp64(acc[2 * j], p_re);
-        const double im = (j & 1) ? oz::scaled_fp64(acc[2 * j + 1], p_im) : oz::scaled(acc[2 * j + 1], p_im);
+      auto store = [&](int j, double re, double im) {
         if constexpr (!PAIRS) {
-          __stcs(s + (rbase | d.ftab[n >> 1]), make_double2(re, im));
+          __stcs(reinterpret_cast<double2*>(row + fo[j]), make_double2(re, im));
         } else if (j & 1) {  // with its neighbour f - 1
-          asm volatile("st.global.cs.v4.f64 [%0], {%1,%2,%3,%4};" ::"l"(s + (rbase | d.ftab[(n >> 1) - 1])),
+          asm volatile("st.global.cs.v4.f64 [%0], {%1,%2,%3,%4};" ::"l"(row + fo[j - 1]),
                        "d"(held.x), "d"(held.y), "d"(re), "d"(im)
                        : "memory");
         } else {
           held = make_double2(re, im);
         }
+      };
+      if (plain) {
+        const uint32_t rh = uint32_t(rem) << 20;
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+          store(j, oz::scaled_plain_fp64(acc[2 * j], rh + fhi[n1 + 2 * j]),
+                oz::scaled_plain_fp64(acc[2 * j + 1], rh + fhi[n1 + 2 * j + 1]));
+      } else {  // results beyond the normal range in some row
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+          store(j, oz::scaled(acc[2 * j], rem + fexp[n1 + 2 * j]),
+                oz::scaled(acc[2 * j + 1], rem + fexp[n1 + 2 * j + 1]));
       }
     }
-    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    // the A slices are rewritten next step: every MMA of this one must be done
-    if (half == 0 && !mbar_wait(&bar[1], phase, kWaitLimit)) {
-      ok = false;
+  };
+
+  uint64_t step = blockIdx.x;
+  uint64_t sb = step_base(d, step);
+  if (step < d.nsteps) {
+    load(sb);
+    em = oz_prepare<ND>(b, err);
+    write_slices(0);
+    if (step + gridDim.x < d.nsteps) {
+      load(advance(sb));
+      em = oz_prepare<ND>(b, err);
+    }
+  }
+  uint32_t phase = 0;
+  for (; step < d.nsteps; step += gridDim.x, phase ^= 1) {
+    // abar orders the other warps' rowexp (it completed before the MMAs began)
+    if (!mbar_wait(&abar, phase, kWaitLimit)) {
       atomicExch(err, 1);
       break;
     }
-    phase ^= 1;
-    sb = ((sb | ~cmask) + gbase) & cmask;
+    const int rem = rowexp[phase][erow];
+    const bool plain =
+        __all_sync(0xFFFFFFFFu, rem == 0 || oz::plain_pow2(rem + flo, rem + ftop));
+    char* const row = reinterpret_cast<char*>(s + (sb | eroff));
+    if (!mbar_wait(&bar[0], phase, kWaitLimit)) {
+      atomicExch(err, 1);
+      break;
+    }
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    recombine(0, row, rem, plain);
+    if (!mbar_wait(&bar[1], phase, kWaitLimit)) {  // every MMA of this step is done
+      atomicExch(err, 1);
+      break;
+    }
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const uint64_t nstep = step + gridDim.x, nstep2 = nstep + gridDim.x;
+    sb = advance(sb);
+    if (nstep < d.nsteps) write_slices(int(phase ^ 1));
+    if (nstep2 < d.nsteps) {
+      const uint64_t b2 = advance(sb);
+      load(b2);
+      // the rows of the step after that into L2 (contiguous runs of 2^lowbits
+      // amplitudes, at most 32 of them, two a warp), so that its loads hit L2
+      if (lane < 2 && 2 * warp + lane < nruns && nstep2 + gridDim.x < d.nsteps)
+        asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(
+                         s + (advance(b2) | d.hitab[2 * warp + lane])),
+                     "r"(run_bytes)
+                     : "memory");
+    }
+    recombine(1, row, rem, plain);
+    if (nstep2 < d.nsteps) em = oz_prepare<ND>(b, err);
   }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   if (warp == 0) {
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem),

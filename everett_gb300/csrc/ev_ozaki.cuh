@@ -18,8 +18,8 @@
 // Diagonals 0..6 are kept, each in its own TMEM accumulator, and
 // recombined in int64 on the integer pipes:
 //     acc = D0 2^40 + D1 2^32 + D2 2^24 + D3 2^16 + D4 2^8 + D5 + round(D6 2^-8),
-// |acc| < 2^61, and y = acc * 2^(E + F_n - 2098) is assembled from acc's
-// bits with one rounding to nearest even.  No step runs on the FP64 pipe.
+// |acc| < 2^61, and y = acc * 2^(E + F_n - 2098) with one rounding to nearest
+// even (the conversion of acc, on the FP64 pipe; the scaling is exact).
 // Error per output, in units u = 2^(E + F_n - 2098): 0.5 from D6's
 // rounding, the dropped pairs i + j >= 7 (at most 2^(7 - 16) * 8 * 2^20 =
 // 128 u, about 2 u for digits of random sign), the truncation of x and W to
@@ -68,18 +68,25 @@ struct Fmt<6> {
   static constexpr int kPow2Bias = 2090;
 };
 
-// M = trunc(x * 2^(1022 + kBits - E)) for the f64 with the given bit halves
-// (E the row's largest biased exponent): 1077 - E for seven digits, 1069 - E
-// for six.  Zero, subnormal values and values 2^53 times below the maximum
-// give 0.
+// M + kBias, M = trunc(x * 2^(1022 + kBits - E)) for the f64 with the given
+// bit halves (E the row's largest biased exponent): 1077 - E for seven digits,
+// 1069 - E for six.  Zero, subnormal values and values 2^53 times below the
+// maximum give M = 0.  One right shift covers every exponent (the 53-bit
+// significand is held two places up for seven digits) and the sign goes in by
+// complement, so that the device runs it without branches.
+template <int ND>
+__host__ __device__ __forceinline__ uint64_t biased(uint32_t hi, uint32_t lo, int E) {
+  constexpr int up = Fmt<ND>::kBits - 53;  // 2 or -6
+  const int e = int((hi >> 20) & 0x7FFu);
+  int d = E - e + (up < 0 ? -up : 0);
+  d = e == 0 || d > 63 ? 63 : d;
+  const uint64_t mant = ((uint64_t((hi & 0xFFFFFu) | 0x100000u) << 32) | lo) << (up > 0 ? up : 0);
+  const uint64_t s = uint64_t(int64_t(int32_t(hi) >> 31));
+  return ((mant >> d) ^ s) - s + Fmt<ND>::kBias;
+}
 template <int ND>
 __host__ __device__ __forceinline__ int64_t fixed(uint32_t hi, uint32_t lo, int E) {
-  const int e = int((hi >> 20) & 0x7FFu);
-  const int sh = E - e + (53 - Fmt<ND>::kBits);
-  if (e == 0 || sh >= 53) return 0;
-  const uint64_t mant = (uint64_t((hi & 0xFFFFFu) | 0x100000u) << 32) | lo;
-  const uint64_t m = sh < 0 ? mant << (-sh) : mant >> sh;
-  return (hi >> 31) ? -int64_t(m) : int64_t(m);
+  return int64_t(biased<ND>(hi, lo, E) - Fmt<ND>::kBias);
 }
 
 // Digit i (0 = most significant) of M in balanced base 256.
@@ -267,18 +274,19 @@ __host__ __device__ __forceinline__ double scaled(int64_t acc, int pow2) {
   return y;
 }
 
+// Whether 2^pow2 times any acc with 1 <= |acc| < 2^62 is a normal f64: then
+// the form below gives scaled()'s value with no branch.
+__host__ __device__ __forceinline__ bool plain_pow2(int lo, int hi) {
+  return lo + 1023 >= 1 && hi + 1085 <= 2046;
+}
 #ifdef __CUDACC__
-// The same value as scaled(), formed on the FP64 pipe: the conversion of acc
-// rounds to nearest even as scaled() does, and a power-of-two scaling that
-// keeps the result normal is exact, an exponent-field add.  The complex128
-// fused pass sends part of its outputs here, where the FP64 pipe is idle
-// while the integer pipes recombine.
-__device__ __forceinline__ double scaled_fp64(int64_t acc, int pow2) {
+// On the FP64 pipe: the conversion of acc rounds to nearest even as scaled()
+// does, and a power-of-two scaling that keeps the result normal is exact, an
+// exponent-field add (pow2 << 20 in the high word; the word of a zero stays).
+__device__ __forceinline__ double scaled_plain_fp64(int64_t acc, uint32_t pow2_hi) {
   const double x = __ll2double_rn(acc);
-  const uint64_t b = uint64_t(__double_as_longlong(x));
-  const int e = int((b >> 52) & 0x7FFu);
-  if (acc == 0 || e + pow2 <= 0 || e + pow2 >= 2047) return acc == 0 ? 0.0 : scalbn(x, pow2);
-  return __longlong_as_double((long long)(b + (uint64_t(int64_t(pow2)) << 52)));
+  const uint32_t hi = uint32_t(__double2hiint(x));
+  return __hiloint2double(int(hi == 0 ? 0u : hi + pow2_hi), __double2loint(x));
 }
 #endif
 

@@ -222,3 +222,54 @@ def test_low_qubit_access_forms(gpu, F, variant):
     dtype = "complex128" if variant.startswith("ozaki") else "complex64"
     got = CudaStateVectorBackend.run(c, dtype=dtype, mode="fused", variant=variant).state().amplitudes()
     assert np.max(np.abs(got - want)) < (1e-12 if dtype == "complex128" else 1e-5)
+
+
+@OZAKI
+@pytest.mark.parametrize("lo", [0, 1, 7])
+def test_ozaki_rows_at_the_ends_of_the_exponent_range(gpu, lo, variant):
+    """Rows whose largest amplitude lies near either end of the f64 range,
+    where results leave the normal numbers: per row within 1e-14 (seven
+    digits) or 2^-39 (six) of its largest amplitude times sqrt(32) (the most
+    it can grow), as for rows of mixed scale, plus 64 times the smallest normal number, which covers subnormal
+    inputs (taken as zero) and the rounding of subnormal results."""
+    from everett_gb300 import State
+    n = 13
+    rng = np.random.default_rng(40 + lo)
+    mask = 31 << lo
+    idx = np.arange(1 << n)
+    key = idx & ~mask
+    order = np.argsort(key, kind="stable")
+    rows = (1 << n) // 32
+    powers = rng.choice([0, -300, -940, -955, -960, -965, -967, -968, -970, -1000, -1015, -1021,
+                         300, 990, 1008, 1012, 1014, 1018], size=rows)
+    amps = np.zeros(1 << n, dtype=np.complex128)
+    vals = (rng.uniform(-1, 1, size=(rows, 32)) + 1j * rng.uniform(-1, 1, size=(rows, 32)))
+    vals = np.ldexp(vals.real, powers[:, None]) + 1j * np.ldexp(vals.imag, powers[:, None])
+    vals[rng.choice(rows, 20, replace=False)] = 0
+    amps[order] = vals.reshape(-1)
+    c = Circuit(n)
+    for q in range(lo, lo + 5):
+        c.rx(q, 0.3 + q).rz(q, 1.1 * q)
+    c.cnot(lo, lo + 4).cz(lo + 1, lo + 3)
+    want = amps.copy()
+    O.apply_ops(c, want, 0, len(c))
+    st = State.from_amplitudes(amps)
+    CudaStateVectorBackend.drive(st, c, 0, mode="fused", variant=variant)
+    g, w = st.amplitudes()[order].reshape(-1, 32), want[order].reshape(-1, 32)
+    diff = np.maximum(np.abs(g.real - w.real), np.abs(g.imag - w.imag)).max(axis=1)
+    rowmax = np.maximum(np.abs(vals.real), np.abs(vals.imag)).max(axis=1)
+    bar = 1e-14 if variant == "ozaki" else 2.0 ** -39
+    assert np.all(diff <= bar * rowmax * np.sqrt(32.0) + 64 * np.finfo(np.float64).tiny)
+    assert np.all(g[rowmax == 0] == 0)
+
+
+@OZAKI
+@pytest.mark.parametrize("n", [19, 20, 21, 22])
+def test_ozaki_several_steps_a_block(gpu, n, variant):
+    """Registers whose blocks run one to seven row steps each (the digits of a
+    step are written while the one before is recombined) against the tile
+    pass: max difference 1e-12, as against the oracle."""
+    c = workloads.random_layers(n, 3, seed=n)
+    want = CudaStateVectorBackend.run(c, dtype="complex128", mode="tiled").state().amplitudes()
+    got = CudaStateVectorBackend.run(c, dtype="complex128", mode="fused", variant=variant).state().amplitudes()
+    assert np.max(np.abs(got - want)) <= 1e-12
