@@ -22,6 +22,7 @@
 #include <vector>
 
 #include "ev_device.cuh"
+#include "ev_bulk.cuh"
 #include "ev_internal.h"
 #include "ev_softfp.cuh"
 
@@ -1368,11 +1369,15 @@ __global__ void __launch_bounds__(kRedThreads, 3)
 // W at its z bits in r's place with the sign of its other bits.  Measured,
 // all 2 n - 1 terms of an Ising chain (Z Z bonds, X sites), a call, one read
 // per X mask -> tiles: complex64 10 qubits 1.33 -> 0.17 ms, 26 qubits 4.91 ->
-// 2.5 ms; complex128 26 qubits 20.1 -> 5.9 ms.
+// 1.91 ms; complex128 26 qubits 20.1 -> 5.8 ms.
 //
-// Bound: instruction issue in complex64 (about 35 instructions per pair and
-// X term; ncu: issue slots 67 % busy, DRAM 15 %), the FP64 pipe in complex128
-// (2 per pair and X term).  Sums as above: complex64 in unnormalised
+// Bound: instruction issue in complex64, the FP64 pipe in complex128 (2 per
+// pair and X term).  In complex64 a pair takes 11 packed operations (both
+// products in the lanes of one register pair) and two loads at fixed offsets
+// where the masks allow it (pauli_slots).  26 qubits, all terms, a call: 2.43 ms with
+// scalar operations and computed offsets, 2.47 packed alone, 2.07 packed
+// with fixed offsets, 1.91 with the tile loaded by asynchronous copies too;
+// complex128 5.89 -> 5.78.  Sums as above: complex64 in unnormalised
 // double-float pairs, flushed to f64 every kPauliRun tiles (8 pairs per
 // thread, term and tile); complex128 in f64.
 constexpr int kPauliEntries = 20;  // terms of a pass: 3 blocks of 72 KiB per SM in complex64
@@ -1389,16 +1394,20 @@ struct PauliEntries {
   int nx, n;  // X terms first
 };
 
+struct F2Lanes;
+struct F64Sum;
 template <typename V>
 struct PauliTile;
 template <>
 struct PauliTile<float2> {
   using Acc = F2;
+  using Sum = F2Lanes;
   static constexpr int K = 12;
 };
 template <>
 struct PauliTile<double2> {
   using Acc = double;
+  using Sum = F64Sum;
   static constexpr int K = 11;
 };
 
@@ -1409,21 +1418,89 @@ __device__ __forceinline__ double flip_if(double v, uint32_t neg) {
   return __longlong_as_double((long long)(uint64_t(__double_as_longlong(v)) ^ (uint64_t(neg) << 63)));
 }
 
-// f += +-Re or +-Im of conj(y) x; the sign rides in the sums' FMAs
+// Two floats in one 64-bit register pair: one instruction rounds both lanes
+// as the scalar operation does.  -1 rides in an FMA in place of a negation.
+__device__ __forceinline__ uint64_t f32x2(float x, float y) {
+  return uint64_t(__float_as_uint(x)) | uint64_t(__float_as_uint(y)) << 32;
+}
+__device__ __forceinline__ float lane_x(uint64_t v) { return __uint_as_float(uint32_t(v)); }
+__device__ __forceinline__ float lane_y(uint64_t v) { return __uint_as_float(uint32_t(v >> 32)); }
+__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
+  uint64_t r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
+  uint64_t r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
+  uint64_t r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+constexpr uint64_t kMinusOne2 = 0xBF800000BF800000ull;
+__device__ __forceinline__ uint64_t sub2(uint64_t a, uint64_t b) { return fma2(b, kMinusOne2, a); }
+
+// A term's sums over a thread's pairs of a tile, which share the sign neg:
+// the accumulator's negated or not, so that the pairs add without one.  The
+// products of the real and of the imaginary parts take a lane each in
+// complex64.
+struct F2Lanes {
+  uint64_t hi, lo;
+  __device__ __forceinline__ F2Lanes(const F2& f, uint32_t neg)
+      : hi(f32x2(flip_if(f.hi, neg), 0.f)), lo(f32x2(flip_if(f.lo, neg), 0.f)) {}
+  __device__ __forceinline__ F2 sum(uint32_t neg) const {
+    F2 g{lane_x(hi), lane_x(lo)};
+    f2_add(g, lane_y(hi), lane_y(lo));
+    return {flip_if(g.hi, neg), flip_if(g.lo, neg)};
+  }
+};
+struct F64Sum {
+  double v;
+  __device__ __forceinline__ F64Sum(double f, uint32_t neg) : v(flip_if(f, neg)) {}
+  __device__ __forceinline__ double sum(uint32_t neg) const { return flip_if(v, neg); }
+};
+
+// f += Re or Im of conj(y) x, products and sums split exactly
 template <int PART>
-__device__ __forceinline__ void pauli_add(F2& f, float2 x, float2 y, uint32_t neg) {
-  const F2 v = PART == 1 ? f2_dot2(y.x, x.x, y.y, x.y) : f2_dot2(y.x, x.y, -y.y, x.x);
-  const float sg = flip_if(1.f, neg);
-  const float s = __fmaf_rn(sg, v.hi, f.hi);
-  const float bp = __fsub_rn(s, f.hi);
-  const float e = __fadd_rn(__fsub_rn(f.hi, __fsub_rn(s, bp)), __fmaf_rn(sg, v.hi, -bp));
-  f = {s, __fadd_rn(__fmaf_rn(sg, v.lo, f.lo), e)};
+__device__ __forceinline__ void pauli_add(F2Lanes& f, float2 x, float2 y) {
+  const uint64_t xx = PART == 1 ? f32x2(x.x, x.y) : f32x2(x.y, x.x);
+  const uint64_t yy = PART == 1 ? f32x2(y.x, y.y) : mul2(f32x2(y.x, y.y), f32x2(1.f, -1.f));
+  const uint64_t p = mul2(yy, xx);
+  const uint64_t ne = fma2(mul2(yy, kMinusOne2), xx, p);  // less the product's error
+  const uint64_t s = add2(f.hi, p);
+  const uint64_t nb = sub2(f.hi, s);
+  const uint64_t e = add2(sub2(f.hi, add2(s, nb)), add2(p, nb));
+  f.hi = s;
+  f.lo = add2(sub2(f.lo, ne), e);
 }
 template <int PART>
-__device__ __forceinline__ void pauli_add(double& f, double2 x, double2 y, uint32_t neg) {
-  const double yx = flip_if(y.x, neg), yy = flip_if(y.y, neg ^ uint32_t(PART == 2));
-  f = __fma_rn(yx, PART == 1 ? x.x : x.y, f);
-  f = __fma_rn(yy, PART == 1 ? x.y : x.x, f);
+__device__ __forceinline__ void pauli_add(F64Sum& f, double2 x, double2 y) {
+  f.v = __fma_rn(y.x, PART == 1 ? x.x : x.y, f.v);
+  f.v = __fma_rn(PART == 1 ? y.y : -y.y, PART == 1 ? x.y : x.x, f.v);
+}
+
+constexpr int kPauliBits = 8;  // log2 kRedThreads
+
+// Full tiles, masks without Z in the bits above kPauliBits: a thread's pairs
+// lie at fixed offsets from two pointers and share their sign.
+//   BIT < 0: the X mask lies among the thread's bits.  The threads t and
+//     t ^ x share the pairs of their slots, one takes the lower half of them
+//     and the other the upper (each slot read once by one thread: no bank is
+//     hit twice).
+//   BIT >= 0: the X mask is bit BIT of the slot: both amplitudes are the
+//     thread's own.
+template <int PART, int BIT, typename V, typename Sum>
+__device__ __forceinline__ void pauli_slots(const V* px, const V* py, Sum& sum) {
+  constexpr int H = (1 << PauliTile<V>::K) / kRedThreads / 2;
+#pragma unroll
+  for (int i = 0; i < H; ++i) {
+    const int r = BIT < 0 ? i : ((i >> (BIT < 0 ? 0 : BIT)) << (BIT + 1)) | (i & ((1 << (BIT < 0 ? 0 : BIT)) - 1));
+    const int q = BIT < 0 ? r : r | (1 << (BIT < 0 ? 0 : BIT));
+    pauli_add<PART>(sum, px[r * kRedThreads], py[q * kRedThreads]);
+  }
 }
 
 // The pairs (j, j ^ xl) of a tile, hb clear in j, kRedThreads at a time: j is
@@ -1432,25 +1509,145 @@ __device__ __forceinline__ void pauli_add(double& f, double2 x, double2 y, uint3
 template <int PART, typename V, typename Acc>
 __device__ __forceinline__ void pauli_pairs(const V* tile, uint32_t pairs, const PauliEntry& e,
                                             uint32_t tneg, Acc& f) {
-  constexpr int kBits = 8;  // log2 kRedThreads
+  using Sum = typename PauliTile<V>::Sum;
+  constexpr uint32_t kThread = kRedThreads - 1;
+  constexpr int kSlotBits = PauliTile<V>::K - kPauliBits;
   const uint32_t xl = e.xl, zl = e.zl, t = threadIdx.x;
   const int hb = e.hb;
+  if (pairs == (1u << (PauliTile<V>::K - 1)) && zl <= kThread &&
+      (xl <= kThread || (xl & (xl - 1)) == 0)) {
+    const V* own = tile + t;
+    if (xl <= kThread) {
+      const uint32_t up = (t >> hb) & 1;
+      const uint32_t off = up << (PauliTile<V>::K - 1);
+      // of the pair (j, j ^ xl), j has bit hb clear; Im changes its sign
+      const uint32_t neg =
+          (tneg ^ uint32_t(__popc((up ? t ^ xl : t) & zl)) ^ (PART == 2 ? up : 0u)) & 1u;
+      Sum sum(f, neg);
+      pauli_slots<PART, -1>(own + off, tile + (t ^ xl) + off, sum);
+      f = sum.sum(neg);
+      return;
+    }
+    const uint32_t neg = (tneg ^ uint32_t(__popc(t & zl))) & 1u;
+    Sum sum(f, neg);
+    switch (hb - kPauliBits) {
+      case 0: pauli_slots<PART, 0>(own, own, sum); break;
+      case 1: pauli_slots<PART, 1>(own, own, sum); break;
+      case 2: pauli_slots<PART, 2>(own, own, sum); break;
+      default:
+        if constexpr (kSlotBits == 4) pauli_slots<PART, 3>(own, own, sum);
+    }
+    f = sum.sum(neg);
+    return;
+  }
   if (t >= pairs) return;
-  const bool low = hb < kBits;  // the bit sits among the thread's bits: steps of 2^9
+  const bool low = hb < kPauliBits;  // the bit sits among the thread's bits: steps of 2^9
   const uint32_t jt = low ? ((t >> hb) << (hb + 1)) | (t & ((1u << hb) - 1)) : t;
-  const uint32_t xt = low ? xl : xl & (kRedThreads - 1);
+  const uint32_t xt = low ? xl : xl & kThread;
   const V* px = tile + jt;
   const V* py = tile + (jt ^ xt);
   const uint32_t nt = tneg ^ uint32_t(__popc(jt & zl));
+  Sum sum(f, 0u);
 #pragma unroll 4
   for (uint32_t r = 0; r < (pairs + kRedThreads - 1) / kRedThreads; ++r) {
-    const uint32_t jr = low ? r << (kBits + 1)
-                            : (((r >> (hb - kBits)) << (hb - kBits + 1)) |
-                               (r & ((1u << (hb - kBits)) - 1)))
-                                  << kBits;
-    const uint32_t yr = low ? jr : jr ^ (xl & ~(kRedThreads - 1u));
-    pauli_add<PART>(f, px[jr], py[yr], (nt ^ uint32_t(__popc(jr & zl))) & 1u);
+    const uint32_t jr = low ? r << (kPauliBits + 1)
+                            : (((r >> (hb - kPauliBits)) << (hb - kPauliBits + 1)) |
+                               (r & ((1u << (hb - kPauliBits)) - 1)))
+                                  << kPauliBits;
+    const uint32_t yr = low ? jr : jr ^ (xl & ~kThread);
+    V y = py[yr];
+    const uint32_t neg = (nt ^ uint32_t(__popc(jr & zl))) & 1u;
+    y.x = flip_if(y.x, neg);
+    y.y = flip_if(y.y, neg);
+    pauli_add<PART>(sum, px[jr], y);
   }
+  f = sum.sum(0u);
+}
+
+// (a, b) <- (a + b, a - b), two pairs of double-floats in lanes
+__device__ __forceinline__ void f2_butterfly2(uint64_t& ahi, uint64_t& alo, uint64_t& bhi, uint64_t& blo) {
+  const uint64_t s = add2(ahi, bhi), d = sub2(ahi, bhi);
+  const uint64_t sb = sub2(s, ahi), db = sub2(d, ahi);
+  const uint64_t se = add2(sub2(ahi, sub2(s, sb)), sub2(bhi, sb));
+  const uint64_t de = sub2(sub2(ahi, sub2(d, db)), add2(bhi, db));
+  const uint64_t ls = add2(alo, blo), ld = sub2(alo, blo);
+  ahi = s;
+  alo = add2(ls, se);
+  bhi = d;
+  blo = add2(ld, de);
+}
+
+// The thread's own amplitudes own[256 r] become W[m], the Walsh-Hadamard
+// transform of |a|^2 over r, in the thread's own slots; each(w) then runs with
+// w(m, f, neg): f += +-W[m].  Slots from size on count as zero.
+template <int R, typename Each>
+__device__ __forceinline__ void pauli_z(float2* own, uint32_t size, Each&& each) {
+  uint64_t hi[R / 2], lo[R / 2];  // W[2 i] and W[2 i + 1] in the lanes
+#pragma unroll
+  for (int i = 0; i < R / 2; ++i) {
+    F2 w[2] = {F2{0.f, 0.f}, F2{0.f, 0.f}};
+#pragma unroll
+    for (int c = 0; c < 2; ++c)
+      if (threadIdx.x + uint32_t(2 * i + c) * kRedThreads < size) {
+        const float2 x = own[(2 * i + c) * kRedThreads];
+        w[c] = f2_dot2(x.x, x.x, x.y, x.y);
+      }
+    f2_butterfly(w[0], w[1]);
+    hi[i] = f32x2(w[0].hi, w[1].hi);
+    lo[i] = f32x2(w[0].lo, w[1].lo);
+  }
+#pragma unroll
+  for (int h = 1; h < R / 2; h <<= 1)
+#pragma unroll
+    for (int i = 0; i < R / 2; ++i)
+      if (!(i & h)) f2_butterfly2(hi[i], lo[i], hi[i + h], lo[i + h]);
+  // slot 2 i holds the high parts of W[2 i] and W[2 i + 1], slot 2 i + 1 the low
+#pragma unroll
+  for (int i = 0; i < R / 2; ++i)
+    if (threadIdx.x + uint32_t(2 * i + 1) * kRedThreads < size) {
+      *reinterpret_cast<uint64_t*>(own + (2 * i) * kRedThreads) = hi[i];
+      *reinterpret_cast<uint64_t*>(own + (2 * i + 1) * kRedThreads) = lo[i];
+    }
+  const float* fl = reinterpret_cast<const float*>(own);
+  if (size >= 2 * kRedThreads)
+    each([&](uint32_t m, F2& f, uint32_t neg) {
+      const float* v = fl + (m >> 1) * (4 * kRedThreads) + (m & 1);
+      f2_add(f, flip_if(v[0], neg), flip_if(v[2 * kRedThreads], neg));
+    });
+  else if (threadIdx.x < size)  // one amplitude a thread: W[0] alone
+    each([&](uint32_t, F2& f, uint32_t neg) {
+      f2_add(f, flip_if(lane_x(hi[0]), neg), flip_if(lane_x(lo[0]), neg));
+    });
+}
+template <int R, typename Each>
+__device__ __forceinline__ void pauli_z(double2* own, uint32_t size, Each&& each) {
+  double w[R];
+#pragma unroll
+  for (int r = 0; r < R; ++r) {
+    w[r] = 0.0;
+    if (threadIdx.x + uint32_t(r) * kRedThreads < size) {
+      const double2 x = own[r * kRedThreads];
+      w[r] = __fma_rn(x.x, x.x, __dmul_rn(x.y, x.y));
+    }
+  }
+#pragma unroll
+  for (int h = 1; h < R; h <<= 1)
+    if (uint32_t(h) * kRedThreads < size)
+#pragma unroll
+      for (int r = 0; r < R; ++r)
+        if (!(r & h)) {
+          const double u = w[r], v = w[r + h];
+          w[r] = __dadd_rn(u, v);
+          w[r + h] = __dsub_rn(u, v);
+        }
+  double* slot = reinterpret_cast<double*>(own);
+#pragma unroll
+  for (int r = 0; r < R; ++r)
+    if (threadIdx.x + uint32_t(r) * kRedThreads < size) slot[r * 2 * kRedThreads] = w[r];
+  if (threadIdx.x < size)
+    each([&](uint32_t m, double& f, uint32_t neg) {
+      f = __dadd_rn(f, flip_if(slot[m * 2 * kRedThreads], neg));
+    });
 }
 
 template <typename V>
@@ -1498,19 +1695,16 @@ __global__ void __launch_bounds__(kRedThreads, 3)
     for (int b = 0; b < plan.ncomp; ++b)
       if ((t >> b) & 1) base |= uint64_t(1) << plan.comp[b];
     __syncthreads();  // the offsets are written; the last tile is no longer read
-    // all loads issued before the first store: a store to the tile could alias
-    // the row offsets, which the compiler would otherwise read again after it
-    V v[R];
+    // the slot's bits and the thread's are disjoint, and so are their offsets
+    if (threadIdx.x < size) {
+      const V* p = a + (base | offs[threadIdx.x >> L] | (threadIdx.x & lowmask));
 #pragma unroll
-    for (int r = 0; r < R; ++r) {
-      const uint32_t l = threadIdx.x + uint32_t(r) * kRedThreads;
-      if (l < size) v[r] = a[base | offs[l >> L] | (l & lowmask)];
+      for (int r = 0; r < R; ++r) {
+        const uint32_t l = uint32_t(r) * kRedThreads;
+        if (l < size) copy_async(tile + threadIdx.x + l, p + offs[l >> L]);
+      }
     }
-#pragma unroll
-    for (int r = 0; r < R; ++r) {
-      const uint32_t l = threadIdx.x + uint32_t(r) * kRedThreads;
-      if (l < size) tile[l] = v[r];
-    }
+    copy_async_wait();
     __syncthreads();
     for (int e = 0; e < en.nx; ++e) {
       const PauliEntry& x = en.e[e];
@@ -1524,53 +1718,16 @@ __global__ void __launch_bounds__(kRedThreads, 3)
     }
     if (en.nx < en.n) {  // Z-only terms
       __syncthreads();   // the tile is overwritten from here on, each thread its own slots
-      Acc w[R];
-#pragma unroll
-      for (int r = 0; r < R; ++r) {
-        const uint32_t l = threadIdx.x + uint32_t(r) * kRedThreads;
-        w[r] = Acc{};
-        if (l < size) {
-          const V x = tile[l];
-          if constexpr (sizeof(V) == 8)
-            w[r] = f2_dot2(x.x, x.x, x.y, x.y);
-          else
-            w[r] = __fma_rn(x.x, x.x, __dmul_rn(x.y, x.y));
-        }
-      }
-#pragma unroll
-      for (int h = 1; h < R; h <<= 1)
-        if (uint32_t(h) * kRedThreads < size)
-#pragma unroll
-          for (int r = 0; r < R; ++r)
-            if (!(r & h)) {
-              if constexpr (sizeof(V) == 8) {
-                f2_butterfly(w[r], w[r + h]);
-              } else {
-                const double u = w[r], v2 = w[r + h];
-                w[r] = __dadd_rn(u, v2);
-                w[r + h] = __dsub_rn(u, v2);
-              }
-            }
-      // W[r] goes into the thread's own slot r of the tile
-      constexpr int kSlot = int(sizeof(V) / sizeof(Acc)) * kRedThreads;
-      Acc* own = reinterpret_cast<Acc*>(tile + threadIdx.x);
-#pragma unroll
-      for (int r = 0; r < R; ++r)
-        if (threadIdx.x + uint32_t(r) * kRedThreads < size) own[r * kSlot] = w[r];
-      if (threadIdx.x < size)
+      pauli_z<R>(tile + threadIdx.x, size, [&](auto&& w) {
         for (int e = en.nx; e < en.n; ++e) {
           const PauliEntry& x = en.e[e];
           const uint32_t neg =
               uint32_t(__popcll(base & x.z) + __popc(threadIdx.x & x.zl & (kRedThreads - 1))) & 1u;
-          const Acc v1 = own[(x.zl / kRedThreads) * kSlot];
-          if constexpr (sizeof(V) == 8) {
-            F2 f = accs[e * kRedThreads];
-            f2_add(f, flip_if(v1.hi, neg), flip_if(v1.lo, neg));
-            accs[e * kRedThreads] = f;
-          } else {
-            accs[e * kRedThreads] = __dadd_rn(accs[e * kRedThreads], flip_if(v1, neg));
-          }
+          Acc f = accs[e * kRedThreads];
+          w(x.zl / kRedThreads, f, neg);
+          accs[e * kRedThreads] = f;
         }
+      });
     }
     if (++run == kPauliRun) {
       flush();

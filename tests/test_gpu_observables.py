@@ -161,3 +161,29 @@ def test_marginal_low_complex64_bits(gpu):
         for row in terms.reshape(-1, 1 << m):
             want = want + row
         assert np.array_equal(st.marginal_low(m), want), m
+
+
+@pytest.mark.parametrize("dtype", ["complex128", "complex64"])
+@pytest.mark.parametrize("n", [11, 12, 14])
+def test_masks_within_a_tile(gpu, n, dtype):
+    """X masks of one and of several bits at every place of a tile (thread
+    bits, one slot bit, several, both), with Z bits nowhere, among the thread
+    bits and among the slot bits, inside and outside the tile, both Y
+    parities: the same bar as above."""
+    rng = np.random.default_rng(100 + n)
+    amps, _, _ = O.run_seeded(workloads.random_layers(n, 3, seed=n + 9), parallel=True)
+    st = State.from_amplitudes(amps, dtype=dtype)
+    ref = np.ascontiguousarray(st.amplitudes())
+    ps = []
+    for width in (1, 2, 3, 5):
+        for _ in range(12):
+            x = np.zeros(n, dtype=bool)
+            x[rng.choice(min(n, 11), width, replace=False)] = True
+            z = rng.integers(0, 2, n).astype(bool) & (rng.uniform(size=n) < rng.choice([0.0, 0.2, 0.6]))
+            ps.append(PauliString(list(x), list(z), bool(rng.integers(0, 2))))
+    for first in range(0, len(ps), 8):  # few masks a call: they share a tile
+        got = st.pauli_expectation(ps[first:first + 8])
+        for p, g in zip(ps[first:first + 8], got):
+            xm, zm = p.masks()
+            want = O.pauli_expectation(ref, xm, zm, p.neg)
+            assert abs(g - want) < 1e-12, (n, dtype, str(p), g, want)
