@@ -38,7 +38,6 @@
 namespace ev {
 namespace oz {
 
-constexpr int kDigits = 7;  // 8-bit digits per value (56 bits)
 constexpr int kK = 64;      // reals per row: 32 amplitudes of a 5-qubit block
 
 // The two digit counts the engine runs.  Seven digits (EV_FUSED_OZAKI) carry
@@ -97,35 +96,11 @@ __host__ __device__ __forceinline__ int digit_of(int64_t M, int i) {
   return int((b >> (8 * (ND - 1 - i))) & 0xFFu) - 128;
 }
 
-// M = trunc(x * 2^(1077 - E)) for the f64 with the given bit halves, where E
-// is the largest biased exponent of its row (or column).  Zero, subnormal
-// values and values 2^53 times below the maximum give 0.
-__host__ __device__ __forceinline__ int64_t fixed55(uint32_t hi, uint32_t lo, int E) {
-  const int e = int((hi >> 20) & 0x7FFu);
-  const int sh = E - e - 2;  // M = mant * 2^(e - E + 2), sh >= -2
-  if (e == 0 || sh >= 53) return 0;
-  const uint64_t mant = (uint64_t((hi & 0xFFFFFu) | 0x100000u) << 32) | lo;
-  const uint64_t m = sh < 0 ? mant << (-sh) : mant >> sh;
-  return (hi >> 31) ? -int64_t(m) : int64_t(m);
-}
-
-// The bias that turns the six low balanced digits into bytes:
-// M + kBias = sum_{k<6} (X_{6-k} + 128) 256^k + X_0 256^6.
-constexpr uint64_t kBias = 0x808080808080ull;
-
-// Digit i (0 = most significant) of M, as an int.
-__host__ __device__ __forceinline__ int digit(int64_t M, int i) {
-  const uint64_t b = uint64_t(M) + kBias;
-  if (i == 0) return int(int32_t(uint32_t(b >> 32)) >> 16);
-  return int((b >> (8 * (6 - i))) & 0xFFu) - 128;
-}
-
 // Recombination of the seven diagonal sums (exact integers held in f32).
 // D0..D3 (|D| <= 2^22) become integers by the magic constant 1.5 * 2^23
 // (the integer sits in the low mantissa bits of D + 1.5 * 2^23); D4 and D5
 // (|D| < 2^23) by a rounding conversion, exact for an integer; D6 by the
 // magic constant 1.5 * 2^31, which leaves round(D6 / 2^8).
-constexpr int kPow2Bias = 2098;  // y = acc * 2^(E + F - kPow2Bias)
 
 __host__ __device__ __forceinline__ float f32_of(uint32_t u) {
   float f;
@@ -147,27 +122,8 @@ __host__ __device__ __forceinline__ float add_rn(float a, float b) {
 #endif
 }
 
-// acc += the contribution of diagonal d whose f32 sum is D.
-template <int d>
-__host__ __device__ __forceinline__ void accumulate(int64_t& acc, float D) {
-  if constexpr (d < 4) {
-    const int32_t v = int32_t(f32_bits(add_rn(D, f32_of(0x4B400000u))) - 0x4B400000u);
-    acc += int64_t(v) * (int64_t(1) << (40 - 8 * d));
-  } else if constexpr (d < 6) {
-#ifdef __CUDA_ARCH__
-    const int32_t v = __float2int_rn(D);
-#else
-    const int32_t v = int32_t(D);  // D is an integer: the conversion is exact
-#endif
-    acc += int64_t(v) * (int64_t(1) << (40 - 8 * d));
-  } else {
-    const int32_t v = int32_t(f32_bits(add_rn(D, f32_of(0x4F400000u))) - 0x4F400000u);
-    acc += int64_t(v);
-  }
-}
-
 // The seven diagonals of one output combined at once, with the same result
-// as accumulate<0..6>: the digit bounds keep three partial sums inside int32,
+// as accumulate_nd<7, 0..6> below: the digit bounds keep three partial sums inside int32,
 //   G3 = 2^8 I0 + I1 (< 2^29),  G2 = 2^8 I2 + I3 (< 2^30),
 //   G1 = 2^8 I4 + I5 + round(D6 / 2^8) (< 2^31),
 // and acc = 2^32 G3 + 2^16 G2 + G1.  The magic constants of the f32-to-int
@@ -193,14 +149,8 @@ __host__ __device__ __forceinline__ int32_t combine_lo(float D4, float D5, float
 __host__ __device__ __forceinline__ int64_t combine_g(int32_t g3, int32_t g2, int32_t g1) {
   return (int64_t(g3) << 32) + (int64_t(g2) << 16) + int64_t(g1);
 }
-__host__ __device__ __forceinline__ int64_t combine7(const float D[7]) {
-  int32_t g3, g2;
-  combine_hi(D[0], D[1], D[2], D[3], g3, g2);
-  return combine_g(g3, g2, combine_lo(D[4], D[5], D[6]));
-}
-
 // acc += the contribution of diagonal d of an ND-digit product whose f32 sum
-// is D (the forms of accumulate<d> above, weights 2^(8 (ND - 2 - d))).
+// is D (weights 2^(8 (ND - 2 - d))).
 template <int ND, int d>
 __host__ __device__ __forceinline__ void accumulate_nd(int64_t& acc, float D) {
   if constexpr (d < 4) {
