@@ -1,0 +1,43 @@
+"""The pass planner (plan_passes, everett_gb300/csrc/ev_tile.cuh) on the host:
+its passes against the rule written out, and its time per gate on long
+circuits against short ones."""
+import shutil
+import subprocess
+from pathlib import Path
+
+import pytest
+
+ROOT = Path(__file__).resolve().parents[1]
+LIBDIR = ROOT / "everett_gb300"
+
+
+@pytest.fixture(scope="module")
+def program(engine, tmp_path_factory):
+    nvcc = shutil.which("nvcc")
+    assert nvcc, "nvcc is required"
+    exe = tmp_path_factory.mktemp("plan") / "test_plan"
+    r = subprocess.run([nvcc, "-gencode", "arch=compute_103a,code=sm_103a", "-std=c++17", "-O2",
+                        "--expt-relaxed-constexpr", "-I", str(LIBDIR / "csrc"),
+                        str(ROOT / "tests" / "cpp" / "test_plan.cu"), "-o", str(exe),
+                        "-L", str(LIBDIR), "-leverett_gb300", "-Xlinker", f"-rpath,{LIBDIR}"],
+                       capture_output=True, text=True)
+    assert r.returncode == 0, r.stdout + r.stderr
+    return exe
+
+
+def test_passes_follow_the_rule(program):
+    r = subprocess.run([str(program), "same"], capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0 and ", 0 differ" in r.stdout, r.stdout + r.stderr
+
+
+def test_planning_is_linear_in_the_gates(program):
+    """400 000 gates take at most four times as long per gate as 10 000 (the
+    longer list leaves the caches; a walk over all that is pending in every
+    pass would take forty times as long), with every qubit in use and with an
+    idle one."""
+    r = subprocess.run([str(program), "time"], capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stdout + r.stderr
+    rows = [line.split() for line in r.stdout.splitlines()]
+    assert len(rows) == 12
+    for n, idle, reorder, short, long in rows:
+        assert float(long) <= 4 * float(short), (n, idle, reorder, short, long)
