@@ -509,6 +509,20 @@ __device__ __forceinline__ void store_four(float2* s, uint64_t rbase, const uint
   }
 }
 
+// Warp 0 of a pass that may start early (early_pass) takes the CTA's TMEM
+// columns before it lets the next pass start.  A CTA that waits for the pass
+// before it with columns in hand then waits for CTAs that have all of theirs;
+// the other way round, passes on two streams could each wait for columns that
+// the other's next pass holds.  One thread's signal counts for its CTA.
+template <int COLS>
+__device__ __forceinline__ void tmem_alloc_then_next(uint32_t* slot) {
+  asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_addr(slot)),
+               "r"(uint32_t(COLS))
+               : "memory");
+  asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
 constexpr int kTcThreads = 256;  // 8 warps: warps w and w+4 share TMEM lane quarter w
 
 template <int KB, int VAR>
@@ -519,8 +533,6 @@ __global__ void __launch_bounds__(kTcThreads, TcShape<KB, VAR>::TC_CTAS)
   constexpr int D = Sh::D, K = Sh::K, ESZ = Sh::ESZ;
   extern __shared__ unsigned char smem_raw[];
   __shared__ FusedDesc d;
-  // the next pass may stage its operands now; it waits below for this one
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   __shared__ __align__(8) uint64_t bar;
   __shared__ uint32_t tmem_slot;
   // aligned by an offset, not by an integer cast: the operands are then
@@ -551,12 +563,9 @@ __global__ void __launch_bounds__(kTcThreads, TcShape<KB, VAR>::TC_CTAS)
     asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_addr(&bar)));
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  if (warp == 0) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
-                     smem_addr(&tmem_slot)),
-                 "r"(uint32_t(Sh::TC_TMEM_COLS)));
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
-  }
+  // the next pass may stage its operands from here on; it waits below for
+  // this one
+  if (warp == 0) tmem_alloc_then_next<Sh::TC_TMEM_COLS>(&tmem_slot);
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
@@ -1128,8 +1137,6 @@ __global__ void __launch_bounds__(kOzThreads, 1)
   constexpr int K = Sh::K;
   extern __shared__ unsigned char smem_raw[];
   __shared__ FusedDesc d;
-  // the next pass may stage its operands now; its workers wait for this one
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   __shared__ __align__(8) uint64_t bar[2];
   __shared__ __align__(8) uint64_t abar;  // a step's A slices written, output half 0 of the one before read
   __shared__ __align__(8) uint64_t tbar;  // a step's output half 1 read
@@ -1168,12 +1175,9 @@ __global__ void __launch_bounds__(kOzThreads, 1)
     mbar_init(&tbar, kOzWorkers / 32);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  if (warp == 0) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
-                     smem_addr(&tmem_slot)),
-                 "r"(uint32_t(Sh::TMEM_COLS)));
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
-  }
+  // the next pass may stage its operands from here on; its workers wait for
+  // this one
+  if (warp == 0) tmem_alloc_then_next<Sh::TMEM_COLS>(&tmem_slot);
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();

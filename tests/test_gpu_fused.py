@@ -273,3 +273,30 @@ def test_ozaki_several_steps_a_block(gpu, n, variant):
     want = CudaStateVectorBackend.run(c, dtype="complex128", mode="tiled").state().amplitudes()
     got = CudaStateVectorBackend.run(c, dtype="complex128", mode="fused", variant=variant).state().amplitudes()
     assert np.max(np.abs(got - want)) <= 1e-12
+
+
+def test_early_passes_on_several_streams(gpu):
+    """Small registers' passes, which may start early, from four threads and
+    states at once (different TMEM needs on one GPU) equal those run alone."""
+    import threading
+    c = workloads.random_layers(16, 6, seed=12)
+    kinds = [("complex64", "tf32x3"), ("complex128", "ozaki"), ("complex64", "bf16x3"),
+             ("complex128", "ozaki6")]
+    alone = [CudaStateVectorBackend.run(c, dtype=d, mode="fused", variant=v).state().amplitudes()
+             for d, v in kinds]
+    wrong = []
+
+    def work(i):
+        d, v = kinds[i]
+        st = CudaStateVectorBackend(16, dtype=d).state()
+        for _ in range(10):
+            CudaStateVectorBackend.run_into(st, c, mode="fused", variant=v)
+            if not np.array_equal(st.amplitudes(), alone[i]):
+                wrong.append(kinds[i])
+
+    threads = [threading.Thread(target=work, args=(i,)) for i in range(len(kinds))]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not wrong
