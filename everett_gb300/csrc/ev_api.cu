@@ -464,7 +464,7 @@ static int create_state(uint64_t n, int32_t dtype, ev_state** out) {
     return fail(EV_ERR_OOM, "cannot allocate %zu bytes for a %llu-qubit state", bytes,
                 (unsigned long long)n);
   }
-  const size_t sb = kMaxRedBlocks * 4 * sizeof(double) + kMaxResults * sizeof(double) + 4 * sizeof(double) +
+  const size_t sb = kPartials * sizeof(double) + kMaxResults * sizeof(double) + 4 * sizeof(double) +
                     64 + 16;
   e = cudaMalloc(&s->scratch_block, sb);
   if (e != cudaSuccess) {
@@ -474,7 +474,7 @@ static int create_state(uint64_t n, int32_t dtype, ev_state** out) {
   }
   char* p = static_cast<char*>(s->scratch_block);
   s->scratch.partials = reinterpret_cast<double*>(p);
-  p += kMaxRedBlocks * 4 * sizeof(double);
+  p += kPartials * sizeof(double);
   s->scratch.result = reinterpret_cast<double*>(p);
   p += kMaxResults * sizeof(double);
   s->scratch.meas = reinterpret_cast<double*>(p);

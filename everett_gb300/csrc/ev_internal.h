@@ -41,13 +41,16 @@ bool debug_enabled();
 // Upper bound on blocks of a reduction grid (partials live in the state's
 // scratch area).
 constexpr int kMaxRedBlocks = 2048;
+// Doubles of the partials: four columns of kMaxRedBlocks blocks, or one wave
+// of Pauli tile blocks (three per SM, 20 columns, up to 273 SMs).
+constexpr int kPartials = 16384;
 // Reduction results that can wait on the device before the host reads them.
 constexpr int kMaxResults = 1024;
 
 // Per-state device scratch: reduction partials, measurement results and the
 // device-resident classical register of a run.
 struct Scratch {
-  double* partials;   // kMaxRedBlocks * 4 doubles
+  double* partials;   // kPartials doubles
   double* result;     // kMaxResults doubles: reduction results
   double* meas;       // 4 doubles: p1, scale, outcome (as double), u
   uint8_t* pred;      // 64 bytes: combined predicates of nested IfClassic

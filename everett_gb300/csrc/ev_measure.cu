@@ -17,6 +17,7 @@
 // terms.  Every reduction accumulates in f64 for both storage types.
 #include <algorithm>
 #include <cmath>
+#include <cstdio>
 #include <cstring>
 #include <mutex>
 #include <vector>
@@ -1380,7 +1381,16 @@ __global__ void __launch_bounds__(kRedThreads, 3)
 // complex128 5.89 -> 5.78.  Sums as above: complex64 in unnormalised
 // double-float pairs, flushed to f64 every kPauliRun tiles (8 pairs per
 // thread, term and tile); complex128 in f64.
-constexpr int kPauliEntries = 20;  // terms of a pass: 3 blocks of 72 KiB per SM in complex64
+//
+// Terms of a pass.  In complex64 three blocks of a full pass share an SM: 32
+// KiB of tile, 2 KiB of accumulators a term, the warps' f64 sums, the row
+// offsets (of 4 bytes: in units of a row) and the 1 KiB that each block is
+// charged.  With offsets of 8 bytes only two fit: the chain above 1.92 ms at
+// 26 qubits and 7.36 at 28, now 1.84 and 6.85.
+constexpr int kPauliEntries = 20;
+constexpr int kPauliRows = 1 << 8;  // 2^(k - L) rows of a full complex64 tile
+static_assert(3 * (32768 + kPauliEntries * (2048 + 64) + 4 * kPauliRows + 1024) <= 228 * 1024,
+              "three blocks per SM");
 
 struct PauliEntry {
   uint64_t z;       // the term's Z mask
@@ -1661,14 +1671,14 @@ __global__ void __launch_bounds__(kRedThreads, 3)
   V* tile = reinterpret_cast<V*>(pt_raw);
   Acc* accs = reinterpret_cast<Acc*>(tile + size) + threadIdx.x;
   __shared__ double wsum[kPauliEntries][kRedThreads / 32];
-  __shared__ uint64_t offs[1 << 8];  // 2^(k - L) row offsets
+  __shared__ uint32_t offs[kPauliRows];  // row offsets in rows of 2^L
   const int tid = int(threadIdx.x), L = plan.L;
   const uint32_t lowmask = (1u << L) - 1;
   for (uint32_t h = threadIdx.x; h < (size >> L); h += kRedThreads) {
     uint64_t o = 0;
     for (int b = 0; b < plan.nH; ++b)
       if ((h >> b) & 1) o |= uint64_t(1) << plan.H[b];
-    offs[h] = o;
+    offs[h] = uint32_t(o >> L);
   }
   for (int e = 0; e < en.n; ++e) accs[e * kRedThreads] = Acc{};
   if (tid < kRedThreads / 32)
@@ -1697,11 +1707,11 @@ __global__ void __launch_bounds__(kRedThreads, 3)
     __syncthreads();  // the offsets are written; the last tile is no longer read
     // the slot's bits and the thread's are disjoint, and so are their offsets
     if (threadIdx.x < size) {
-      const V* p = a + (base | offs[threadIdx.x >> L] | (threadIdx.x & lowmask));
+      const V* p = a + (base | uint64_t(offs[threadIdx.x >> L]) << L | (threadIdx.x & lowmask));
 #pragma unroll
       for (int r = 0; r < R; ++r) {
         const uint32_t l = uint32_t(r) * kRedThreads;
-        if (l < size) copy_async(tile + threadIdx.x + l, p + offs[l >> L]);
+        if (l < size) copy_async(tile + threadIdx.x + l, p + (uint64_t(offs[l >> L]) << L));
       }
     }
     copy_async_wait();
@@ -1822,7 +1832,10 @@ static int launch_pauli_tile(const ev_state* s, const PauliLaunch& p, const uint
   if (ntiles > uint64_t(s->num_sms))
     EV_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_pauli_tile<V>, kRedThreads, smem));
   uint64_t nb = uint64_t(s->num_sms) * uint64_t(per_sm < 1 ? 1 : per_sm);
-  nb = std::min(std::min(nb, ntiles), uint64_t(kMaxRedBlocks * 4 / p.n));
+  nb = std::min(std::min(nb, ntiles), uint64_t(kPartials / p.n));
+  if (debug_enabled())
+    fprintf(stderr, "[ev] k_pauli_tile %d terms (%d X), smem %zu, %d CTAs/SM, grid %llu\n", p.n, p.nx, smem,
+            per_sm, (unsigned long long)nb);
   k_pauli_tile<V><<<unsigned(nb), kRedThreads, smem, s->stream>>>(static_cast<const V*>(s->amps),
                                                                    ntiles, plan, en,
                                                                    s->scratch.partials);

@@ -6,6 +6,11 @@ Bars: 1e-12 absolute in complex128 and, in complex64, against the oracle on
 the same complex64 amplitudes (double-float sums on the FP32 pipe); the
 stabilizer generators of a Clifford state have expectation 1 to 1e-12
 (tests/stabilizer.rs:13-25 uses the statevector the same way)."""
+import os
+import subprocess
+import sys
+from pathlib import Path
+
 import numpy as np
 import pytest
 
@@ -14,6 +19,7 @@ from everett_gb300 import Circuit, algorithms, CudaStateVectorBackend, PauliStri
 from everett_gb300.error import QubitOutOfRange
 
 pytestmark = pytest.mark.gpu
+ROOT = Path(__file__).resolve().parents[1]
 
 
 def random_paulis(rng, n, count):
@@ -187,3 +193,33 @@ def test_masks_within_a_tile(gpu, n, dtype):
             xm, zm = p.masks()
             want = O.pauli_expectation(ref, xm, zm, p.neg)
             assert abs(g - want) < 1e-12, (n, dtype, str(p), g, want)
+
+
+FULL_PASS = """
+import numpy as np
+from everett_gb300 import Gate1, State
+n = 22
+st = State.zero(n, "complex64")
+for q in range(n):
+    st.apply_1q(q, Gate1.ry(0.1 + 0.05 * q))
+chain = ["I" * q + "X" + "I" * (n - q - 1) for q in range(12)]
+chain += ["I" * q + "ZZ" + "I" * (n - q - 2) for q in range(8)]
+angle = 0.1 + 0.05 * np.arange(n)
+want = list(np.sin(angle[:12])) + list(np.cos(angle[:8]) * np.cos(angle[1:9]))
+print(np.max(np.abs(st.pauli_expectation(chain) - want)))
+"""
+
+
+def test_full_pauli_passes_fill_the_gpu(gpu):
+    """A complex64 tile pass of 20 terms, X and Z, has three blocks on every
+    SM in one wave, and the values hold there (22 rotations in single
+    precision, each within 3 units of 2^-24: 8e-6 of an expectation)."""
+    import torch
+    r = subprocess.run([sys.executable, "-c", FULL_PASS], capture_output=True, text=True, timeout=300,
+                       env=dict(os.environ, EV_DEBUG="1"), cwd=ROOT)
+    assert r.returncode == 0, r.stderr
+    assert float(r.stdout) < 1e-5
+    lines = [x for x in r.stderr.splitlines() if "k_pauli_tile 20 terms" in x]
+    assert len(lines) == 1 and " 3 CTAs/SM" in lines[0], r.stderr
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    assert lines[0].endswith(f"grid {min(3 * sms, 1 << (22 - 12))}"), lines
