@@ -20,6 +20,7 @@
 #include <cstdio>
 #include <cstring>
 #include <mutex>
+#include <tuple>
 #include <vector>
 
 #include "ev_device.cuh"
@@ -1889,38 +1890,75 @@ static int launch_pauli_group(const ev_state* s, const PauliLaunch& p, const uin
   return EV_OK;
 }
 
-// Packs the terms into reads of the state: tile passes of up to
-// kPauliEntries terms for X parts that fit a tile's qubits (with the four
-// lowest) and for more Z-only terms than a group pass takes; group passes for
-// the rest, and for X parts that all agree (one group by itself: 26 qubits,
-// complex64, 0.14 ms against 0.20 from tiles; two X masks 0.28 against 0.25).
+// Packs the terms into reads of the state.  Terms that share their X mask and
+// Y parity share their pairs in a group pass, which costs nearly the same for
+// one term as for kPauliTerms; a tile pass serves any X masks that fit its
+// qubits (with the four lowest) but forms every term's products anew.  So
+// group_from or more of one group take group passes, the rest tile passes of
+// up to kPauliEntries terms, as do more Z-only terms than a group pass takes.
+//
+// Where the line lies: a group pass is latency-bound below 23 qubits, and a
+// tile pass's cost goes with its terms.  Two X masks of g terms each, a call,
+// us, group passes / one tile pass:
+//   complex64, 21 qubits: g = 8 228 / 223; 22: 6 190 / 191, 8 233 / 251; 23: 3
+//   150 / 135, 4 161 / 170; 24: 2 148 / 146, 3 166 / 191, 8 266 / 426; 25: 1
+//   171 / 156, 2 189 / 224; 26: 1 259 / 249, 2 280 / 373, 8 425 / 1142
+//   complex128, 22: 8 333 / 307; 23: 4 264 / 241, 6 308 / 331; 24: 4 409 /
+//   353, 6 449 / 518, 8 485 / 667; 26: 3 1048 / 837, 4 1077 / 1098, 8 1212 /
+//   2090; 28: 3 3832 / 3058, 4 3912 / 4017
+static int group_from(int dtype, int n) {
+  const int never = kPauliTerms + 1;
+  if (dtype == EV_C128) return n >= 26 ? 4 : n >= 24 ? 5 : n == 23 ? 6 : never;
+  return n >= 25 ? 2 : n == 24 ? 3 : n == 23 ? 4 : n == 22 ? 7 : never;
+}
+
 static std::vector<PauliLaunch> plan_pauli(const ev_state* s, const uint64_t* x_masks,
                                            const uint64_t* z_masks, uint64_t count) {
   const int n = int(s->n);
   const int k = std::min(n, s->dtype == EV_C128 ? PauliTile<double2>::K : PauliTile<float2>::K);
   const uint64_t low = (uint64_t(1) << std::min(4, k)) - 1;
-  std::vector<uint64_t> wide, fits, zonly;  // terms by kind, in order
-  for (uint64_t t = 0; t < count; ++t)
-    (x_masks[t] == 0 ? zonly : __builtin_popcountll(x_masks[t] | low) <= k ? fits : wide).push_back(t);
   std::vector<PauliLaunch> out;
   auto same_group = [&](uint64_t t, uint64_t u) {
     return x_masks[t] == x_masks[u] && pauli_part(x_masks[t], z_masks[t]) == pauli_part(x_masks[u], z_masks[u]);
   };
-  // group passes of a list whose terms share nothing in general
-  auto add_groups = [&](const std::vector<uint64_t>& list) {
-    std::vector<char> used(list.size(), 0);
-    for (size_t i = 0; i < list.size(); ++i) {
-      if (used[i]) continue;
-      PauliLaunch p;
-      for (size_t j = i; j < list.size() && p.n < kPauliTerms; ++j)
-        if (!used[j] && same_group(list[i], list[j])) {
-          used[j] = 1;
-          p.terms[p.n++] = list[j];
-        }
-      p.nx = x_masks[list[i]] ? p.n : 0;
-      out.push_back(p);
-    }
+  auto add_group = [&](const uint64_t* t, int terms) {
+    PauliLaunch p;
+    p.n = terms;
+    p.nx = x_masks[*t] ? terms : 0;
+    std::copy(t, t + terms, p.terms);
+    out.push_back(p);
   };
+  // terms by group, the groups by their first term
+  std::vector<uint64_t> order(count), first(count), zonly, fits;
+  for (uint64_t t = 0; t < count; ++t) order[t] = t;
+  std::sort(order.begin(), order.end(), [&](uint64_t t, uint64_t u) {
+    const int pt = pauli_part(x_masks[t], z_masks[t]), pu = pauli_part(x_masks[u], z_masks[u]);
+    return std::tie(x_masks[t], pt, t) < std::tie(x_masks[u], pu, u);
+  });
+  for (uint64_t i = 0; i < count; ++i)
+    first[order[i]] = i > 0 && same_group(order[i], order[i - 1]) ? first[order[i - 1]] : order[i];
+  std::sort(order.begin(), order.end(), [&](uint64_t t, uint64_t u) {
+    return std::tie(first[t], t) < std::tie(first[u], u);
+  });
+  for (uint64_t i = 0; i < count;) {
+    uint64_t e = i;
+    while (e < count && first[order[e]] == first[order[i]]) ++e;
+    const uint64_t x = x_masks[order[i]];
+    if (x == 0) {
+      zonly.assign(order.begin() + ptrdiff_t(i), order.begin() + ptrdiff_t(e));
+      i = e;
+      continue;
+    }
+    const int from = __builtin_popcountll(x | low) <= k ? group_from(s->dtype, n) : 1;
+    for (; i < e; i += uint64_t(kPauliTerms)) {
+      const int terms = int(std::min<uint64_t>(e - i, kPauliTerms));
+      if (terms >= from)
+        add_group(&order[i], terms);
+      else
+        fits.insert(fits.end(), order.begin() + ptrdiff_t(i), order.begin() + ptrdiff_t(i) + terms);
+    }
+    i = e;
+  }
   while (!fits.empty()) {
     PauliLaunch p;
     p.tile = true;
@@ -1940,7 +1978,6 @@ static std::vector<PauliLaunch> plan_pauli(const ev_state* s, const uint64_t* x_
     out.push_back(p);
     fits.swap(rest);
   }
-  add_groups(wide);
   // Z-only terms join the tile passes with the most room (their transform
   // is one cost per pass), then fill passes of their own
   std::vector<PauliLaunch*> room;
@@ -1957,7 +1994,7 @@ static std::vector<PauliLaunch> plan_pauli(const ev_state* s, const uint64_t* x_
     while (p.n < kPauliEntries && at < zonly.size()) p.terms[p.n++] = zonly[at++];
     out.push_back(p);
   }
-  add_groups(std::vector<uint64_t>(zonly.begin() + ptrdiff_t(at), zonly.end()));
+  if (at < zonly.size()) add_group(&zonly[at], int(zonly.size() - at));
   for (PauliLaunch& p : out)  // fill T up to k with the lowest unused qubits
     for (int q = 0; p.tile && q < n && __builtin_popcountll(p.set) < k; ++q) p.set |= uint64_t(1) << q;
   return out;

@@ -223,3 +223,65 @@ def test_full_pauli_passes_fill_the_gpu(gpu):
     assert len(lines) == 1 and " 3 CTAs/SM" in lines[0], r.stderr
     sms = torch.cuda.get_device_properties(0).multi_processor_count
     assert lines[0].endswith(f"grid {min(3 * sms, 1 << (22 - 12))}"), lines
+
+
+SHARED = """
+import numpy as np
+import sys
+from everett_gb300 import Gate1, PauliString, State
+n, dtype, masks, g = int(sys.argv[1]), sys.argv[2], 2, int(sys.argv[3])
+st = State.zero(n, dtype)
+for q in range(n):
+    st.apply_1q(q, Gate1.ry(0.1 + 0.05 * q))
+rng = np.random.default_rng(3)
+ps, want = [], []
+for m in range(masks):
+    for t in range(g):
+        z = rng.integers(0, 2, n).astype(bool)
+        z[m + 3] = False
+        x = np.arange(n) == m + 3
+        ps.append(PauliString(list(x), list(z)))
+        a = 0.1 + 0.05 * np.arange(n)
+        want.append(np.prod(np.where(x, np.sin(a), np.where(z, np.cos(a), 1.0))))
+print(np.max(np.abs(st.pauli_expectation(ps) - np.array(want))))
+"""
+
+
+@pytest.mark.parametrize("n,dtype,g,tiles", [
+    (22, "complex64", 6, 1), (22, "complex64", 7, 0), (23, "complex64", 3, 1), (23, "complex64", 4, 0),
+    (24, "complex64", 2, 1), (24, "complex64", 3, 0), (25, "complex64", 1, 1), (25, "complex64", 2, 0),
+    (25, "complex64", 8, 0), (22, "complex128", 8, 1), (23, "complex128", 5, 1),
+    (23, "complex128", 6, 0), (24, "complex128", 4, 1), (24, "complex128", 5, 0),
+    (24, "complex128", 8, 0)])
+def test_terms_of_one_mask_share_their_pairs(gpu, n, dtype, g, tiles):
+    """Two X masks of g terms each on a large register: from the rule's line
+    on each mask takes one read that forms its pairs once, below it both go
+    to one tile pass.  Values as above (complex64: n rotations of 2^-22.4
+    each, twice)."""
+    r = subprocess.run([sys.executable, "-c", SHARED, str(n), dtype, str(g)], capture_output=True,
+                       text=True, timeout=300, env=dict(os.environ, EV_DEBUG="1"), cwd=ROOT)
+    assert r.returncode == 0, r.stderr
+    assert float(r.stdout) < (1e-12 if dtype == "complex128" else 1e-5)
+    assert sum("k_pauli_tile" in x for x in r.stderr.splitlines()) == tiles, r.stderr
+
+
+@pytest.mark.parametrize("dtype", ["complex128", "complex64"])
+def test_more_terms_than_results_wait_on_the_device(gpu, dtype):
+    """2500 terms in one call, whose sums come back in several copies: masks
+    of one term, of many (both Y parities), wide ones and Z strings, shuffled."""
+    n = 13
+    rng = np.random.default_rng(8)
+    amps, _, _ = O.run_seeded(workloads.random_layers(n, 3, seed=4), parallel=True)
+    st = State.from_amplitudes(amps, dtype=dtype)
+    ref = np.ascontiguousarray(st.amplitudes())
+    xs = [rng.uniform(size=n) < f for f in (0.1, 0.2, 0.3, 1.0) for _ in range(40)]
+    ps = random_paulis(rng, n, 300)
+    ps += [PauliString([False] * n, rng.integers(0, 2, n).astype(bool)) for _ in range(200)]
+    ps += [PauliString(xs[int(rng.integers(len(xs)))], rng.integers(0, 2, n).astype(bool),
+                       bool(rng.integers(0, 2))) for _ in range(2000)]
+    ps = [ps[i] for i in rng.permutation(len(ps))]
+    got = st.pauli_expectation(ps)
+    for p, g in zip(ps, got):
+        xm, zm = p.masks()
+        want = O.pauli_expectation(ref, xm, zm, p.neg)
+        assert abs(g - want) < 1e-12, (dtype, str(p), g, want)
