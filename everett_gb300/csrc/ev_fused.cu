@@ -45,6 +45,7 @@
 
 #include "ev_bulk.cuh"
 #include "ev_device.cuh"
+#include "ev_fuse.h"
 #include "ev_internal.h"
 #include "ev_ozaki.cuh"
 
@@ -85,67 +86,6 @@ static uint64_t op_qubits(const ev_circuit* c, const ev_op& op) {
   if (op.kind == EV_OP_CONTROLLED)
     for (uint32_t j = 0; j < op.nctrl; ++j) m |= uint64_t(1) << c->ctrl_pool[op.ctrl_off + j];
   return m;
-}
-
-// The planner's complex arithmetic, written out on rows of interleaved
-// doubles: std::complex multiplies through a library call that checks for
-// NaN, which made fusing the blocks of a 16-qubit run take longer than
-// running them.
-// (x, y) <- (m0 x + m1 y, m2 x + m3 y) over two rows of n complex values
-static void mix_rows(const double* m, double* x, double* y, int n) {
-  for (int i = 0; i < 2 * n; i += 2) {
-    const double xr = x[i], xi = x[i + 1], yr = y[i], yi = y[i + 1];
-    x[i] = (m[0] * xr - m[1] * xi) + (m[2] * yr - m[3] * yi);
-    x[i + 1] = (m[0] * xi + m[1] * xr) + (m[2] * yi + m[3] * yr);
-    y[i] = (m[4] * xr - m[5] * xi) + (m[6] * yr - m[7] * yi);
-    y[i + 1] = (m[4] * xi + m[5] * xr) + (m[6] * yi + m[7] * yr);
-  }
-}
-
-// Left-multiplies U (d x d, local bit i <-> F[i]) by one gate record: the
-// gate combines whole rows of U.
-static void apply_to_unitary(const ev_circuit* c, const ev_op& op, const std::vector<int>& F,
-                             std::vector<cd>* U) {
-  const int d = int(1u << F.size());
-  auto loc = [&](uint64_t q) { return int(std::find(F.begin(), F.end(), int(q)) - F.begin()); };
-  auto row = [&](int r) { return reinterpret_cast<double*>(U->data() + size_t(r) * d); };
-  if (op.kind == EV_OP_APPLY2) {
-    const int ba = 1 << loc(op.q0), bb = 1 << loc(op.q1);
-    const Kind2 kind = classify2(op.m);
-    double out[4][2 * 64];
-    for (int base = 0; base < d; ++base) {
-      if (base & (ba | bb)) continue;
-      double* in[4] = {row(base), row(base | bb), row(base | ba), row(base | ba | bb)};
-      if (kind == K2_CNOT || kind == K2_SWAP) {
-        std::swap_ranges(in[2], in[2] + 2 * d, kind == K2_CNOT ? in[3] : in[1]);
-        continue;
-      }
-      if (kind == K2_CZ) {
-        for (int i = 0; i < 2 * d; ++i) in[3][i] = -in[3][i];
-        continue;
-      }
-      for (int r = 0; r < 4; ++r) {
-        std::fill(out[r], out[r] + 2 * d, 0.0);
-        for (int k = 0; k < 4; ++k) {
-          const double re = op.m[2 * (4 * r + k)], im = op.m[2 * (4 * r + k) + 1];
-          if (re == 0.0 && im == 0.0) continue;
-          const double* v = in[k];
-          for (int i = 0; i < 2 * d; i += 2) {
-            out[r][i] += re * v[i] - im * v[i + 1];
-            out[r][i + 1] += re * v[i + 1] + im * v[i];
-          }
-        }
-      }
-      for (int r = 0; r < 4; ++r) std::copy(out[r], out[r] + 2 * d, in[r]);
-    }
-    return;
-  }
-  const int tb = 1 << loc(op.q0);
-  int cmask = 0;
-  if (op.kind == EV_OP_CONTROLLED)
-    for (uint32_t j = 0; j < op.nctrl; ++j) cmask |= 1 << loc(c->ctrl_pool[op.ctrl_off + j]);
-  for (int i0 = 0; i0 < d; ++i0)
-    if (!(i0 & tb) && (i0 & cmask) == cmask) mix_rows(op.m, row(i0), row(i0 | tb), d);
 }
 
 // Greedy fusion: each block starts at the first pending record and takes
