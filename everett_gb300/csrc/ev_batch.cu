@@ -46,6 +46,7 @@
 
 #include <sys/stat.h>
 
+#include "ev_parallel.h"
 #include "ev_stage.cuh"
 #include "ev_tile.cuh"
 
@@ -852,16 +853,9 @@ static int batch_once(Arena& A, const ev_batch_circuit* items, uint64_t count, i
                   (unsigned long long)items[i].circuit.num_qubits);
   // plan all circuits (in parallel)
   std::vector<CircPlan> cp(count);
-  {
-    const unsigned hw = std::max(1u, std::min(16u, std::thread::hardware_concurrency()));
-    std::vector<std::thread> pool;
-    for (unsigned w = 0; w < hw; ++w)
-      pool.emplace_back([&, w] {
-        for (uint64_t i = w; i < count; i += hw)
-          plan_circuit(&items[i].circuit, kmax, dtype == EV_C64, window, &cp[i]);
-      });
-    for (auto& th : pool) th.join();
-  }
+  parallel_for(count, std::min(16u, std::thread::hardware_concurrency()), [&](uint64_t i) {
+    plan_circuit(&items[i].circuit, kmax, dtype == EV_C64, window, &cp[i]);
+  });
   // layout
   std::vector<BatchCirc> circs(count);
   uint64_t amps = 0, tree = 0, uni = 0, shots = 0, nplans = 0, nops = 0, nmats = 0, ncl = 0;
