@@ -486,12 +486,14 @@ __device__ __forceinline__ void xoshiro_step(uint64_t (&s)[4]) {
 }
 
 __global__ void __launch_bounds__(256)
-    k_batch_uniforms(const BatchCirc* __restrict__ circs, double* __restrict__ uni) {
+    k_batch_uniforms(const BatchCirc* __restrict__ circs, unsigned per, double* __restrict__ uni) {
+  // `per` blocks a circuit along the grid's x: y ends at 65535 blocks, 4.3e9
+  // draws, which one circuit's shots can pass
   __shared__ ulonglong2 cols[256][2];  // column j of the current matrix
-  const BatchCirc& c = circs[blockIdx.x];
+  const BatchCirc& c = circs[blockIdx.x / per];
   const uint64_t total = c.shots * c.n;
   const uint64_t chunks = (total + kChunk - 1) / kChunk;
-  const uint64_t first = uint64_t(blockIdx.y) * 256;
+  const uint64_t first = uint64_t(blockIdx.x % per) * 256;
   if (first >= chunks) return;  // uniform across the block
   const uint64_t mine = first + threadIdx.x;
   const uint64_t last = min(first + 255, chunks - 1);  // the highest chunk of the block
@@ -979,10 +981,11 @@ static int batch_once(Arena& A, const ev_batch_circuit* items, uint64_t count, i
   EV_CUDA(cudaEventRecord(A.e0, A.stream));
   uint64_t most = 0;  // draws of one circuit
   for (uint64_t i = 0; i < count; ++i) most = std::max(most, circs[i].shots * circs[i].n);
-  const uint64_t per_block = uint64_t(kChunk) * 256;
-  if (most > 0)
-    k_batch_uniforms<<<dim3(unsigned(count), unsigned((most + per_block - 1) / per_block)), 256, 0,
-                       A.stream>>>(args.circs, args.uni);
+  const uint64_t per_block = uint64_t(kChunk) * 256, per = (most + per_block - 1) / per_block;
+  const uint64_t at_once = per > 0 ? 0x7FFFFFFFu / per : 0;  // circuits of a launch
+  for (uint64_t i = 0; per > 0 && i < count; i += at_once)
+    k_batch_uniforms<<<unsigned(std::min(at_once, count - i) * per), 256, 0, A.stream>>>(
+        args.circs + i, unsigned(per), args.uni);
   // every CTA of the persistent grid must be resident (items wait on each other)
   const unsigned grid = unsigned(sms * per_sm);
   if (debug_enabled())
