@@ -1,10 +1,10 @@
 // ev_stage.cuh -- runs of complex64 gate records applied to amplitudes held
-// in registers, 16 a thread (tiles of 2^12 amplitudes and more, in the tile
-// pass and the batched runner).
+// in registers, 16 a thread (tiles of 2^12 amplitudes and more in the tile
+// pass, of 2^11 and more in the batched runner).
 //
-// A stage names four positions of the tile; each thread gathers the amplitudes that agree outside them,
-// applies every record of the stage to them in circuit order and scatters
-// them.  A record needs its moved positions (1-qubit target, CNOT target,
+// A stage names four positions of the tile; each thread gathers the
+// amplitudes that agree outside them, applies every record of the stage to
+// them in circuit order and scatters them.  A record needs its moved positions (1-qubit target, CNOT target,
 // both of a SWAP or a dense 4x4) among them; a position it only reads (a control, the bits a
 // diagonal entry depends on) may also be a bit of the thread's index, where
 // it selects threads or the entry.  So a whole ladder of controlled phases

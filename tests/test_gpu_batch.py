@@ -19,6 +19,7 @@ import oracle as O
 from everett_gb300 import (Apply1, Circuit, Gate1, IfClassic, Measure, Rng, algorithms, batch,
                            workloads)
 from everett_gb300.error import DeviceTimeout, InvalidArgument
+from test_gpu_tile_sizes import every_record_kind
 
 pytestmark = pytest.mark.gpu
 
@@ -216,3 +217,59 @@ def test_batch_bounded_wait_reports_timeout(gpu):
     for c, r in zip(circs, res):
         want, _, _ = O.run_seeded(c, 0)
         assert np.array_equal(r.amplitudes, want)
+
+
+STAGED = pytest.mark.parametrize("tile_bits,threads", [(11, 256), (11, 512), (12, 256), (13, 256),
+                                                       (13, 512), (14, 256)])
+
+
+def close64(got, want):
+    """complex64 amplitudes to the tile pass's bar, up to the norm that gates
+    which are not unitary leave."""
+    got, want = got / np.linalg.norm(got), want / np.linalg.norm(want)
+    return np.max(np.abs(got - want)) < 1e-5
+
+
+@STAGED
+def test_staged_batch_every_record_kind(gpu, tile_bits, threads):
+    """complex64 tiles of 2^11 amplitudes and more run in stages of 16
+    amplitudes a thread: every record kind, on registers inside a tile (in
+    the kernel compiled with stages, below 2^11 without them), of a tile and
+    beyond one, with controls outside the tile and runs longer than the
+    record window; shots from the returned amplitudes."""
+    circs = [every_record_kind(n, 10 * n + tile_bits, 260) for n in (4, 7, 10, 11, 12, 13, 14, 16)]
+    circs += tfim_mix(8, 3, 16, seed=tile_bits, smin=3, smax=8)
+    res, stats = batch.run_batch(circs, seeds=range(len(circs)), shots=150, dtype="complex64",
+                                 tile_bits=tile_bits, threads=threads, return_states=True)
+    assert (stats["tile_bits"], stats["threads"]) == (tile_bits, threads)
+    for i, (c, r) in enumerate(zip(circs, res)):
+        want, _, rc = O.run_seeded(c, 0)
+        assert rc == 0
+        assert close64(r.amplitudes, want), (i, c.num_qubits())
+        assert np.array_equal(r.shots, O.sample_tree(np.ascontiguousarray(r.amplitudes), i, 150)), i
+
+
+@STAGED
+def test_staged_batch_classical_control(gpu, tile_bits, threads):
+    """Measurements and classical control between staged records: the
+    circuits above, and registers of 11 qubits up to the tile with every
+    record kind before and after a measurement and under IfClassic."""
+    circs = classical_mix(9) + window_edge_circuits()
+    for n in range(11, tile_bits + 1):
+        c = Circuit.with_classical(n, 2)
+        c.compose(every_record_kind(n, n, 40)).measure(1, 0).measure(n - 1, 1)
+        for t, q in ((Gate1.ry(0.9), 3), (Gate1.rz(0.4), 0), (Gate1.rx(1.3), n - 2)):
+            c.if_classic(0, Apply1(t, q))
+            c.if_classic(1, IfClassic(0, Apply1(t, (q + 5) % n)))
+        c.x_if(1, 4).compose(every_record_kind(n, n + 50, 40))
+        circs.append(c)
+    run_seeds = [3 + 5 * i for i in range(len(circs))]
+    res, _ = batch.run_batch(circs, seeds=range(len(circs)), shots=100, dtype="complex64",
+                             tile_bits=tile_bits, threads=threads, return_states=True,
+                             run_seeds=run_seeds)
+    for i, (c, r) in enumerate(zip(circs, res)):
+        want, bits, rc = O.run_seeded(c, run_seeds[i])
+        assert rc == 0
+        assert r.classical == bits, i
+        assert close64(r.amplitudes, want), (i, c.num_qubits())
+        assert np.array_equal(r.shots, O.sample_tree(np.ascontiguousarray(r.amplitudes), i, 100)), i
