@@ -37,6 +37,7 @@
 #include <cstdio>
 #include <cstdlib>
 #include <fstream>
+#include <map>
 #include <mutex>
 #include <sstream>
 #include <string>
@@ -753,9 +754,31 @@ std::string cache_path() {
   return "everett_gb300_autotune.txt";
 }
 
-std::string batch_key(const ev_batch_circuit* items, uint64_t count, int dtype) {
-  // (amplitude type, qubit-count histogram in 4-qubit buckets, share of
-  // 2-qubit records in tenths)
+// The device's name as one word (queried once: it takes milliseconds).
+std::string device_name(int dev) {
+  static std::mutex mu;
+  static std::map<int, std::string> known;
+  std::lock_guard<std::mutex> lock(mu);
+  std::string& name = known[dev];
+  if (name.empty()) {
+    cudaDeviceProp prop{};
+    if (cudaGetDeviceProperties(&prop, dev) == cudaSuccess) name = prop.name;
+    for (char& c : name)
+      if (c == ' ') c = '_';
+    if (name.empty()) name = "gpu";
+  }
+  return name;
+}
+
+// Raised when a kernel's best shapes move: a record tuned with another
+// revision's kernels is not read (records without one are the first's).
+constexpr int kBatchRevision = 2;
+
+// (revision, device, tile bits and threads that the caller fixed, amplitude
+// type, qubit-count histogram in 4-qubit buckets, share of 2-qubit records in
+// tenths)
+std::string batch_key(const ev_batch_circuit* items, uint64_t count, int dtype, int kbits, int threads,
+                      const std::string& device) {
   int hist[16] = {0};
   uint64_t ops = 0, two = 0;
   for (uint64_t i = 0; i < count; ++i) {
@@ -767,7 +790,8 @@ std::string batch_key(const ev_batch_circuit* items, uint64_t count, int dtype) 
     }
   }
   std::ostringstream k;
-  k << (dtype == EV_C128 ? "c128" : "c64") << ":n";
+  k << "r" << kBatchRevision << ":" << device << ":k" << std::max(kbits, 0) << "t" << std::max(threads, 0)
+    << ":" << (dtype == EV_C128 ? "c128" : "c64") << ":n";
   for (int b = 0; b < 16; ++b)
     if (hist[b]) k << b * 4 << "-" << b * 4 + 3 << "x" << (hist[b] * 10 + int(count) / 2) / int(count) << ",";
   k << ":2q" << (ops ? (two * 10 + ops / 2) / ops : 0);
@@ -799,6 +823,10 @@ void cache_store(const std::string& key, int kbits, int threads) {
 // CTA with a 128 KiB tile.
 int default_tile_bits_batch(int dtype) { return dtype == EV_C128 ? 12 : 13; }
 int max_tile_bits(int dtype) { return dtype == EV_C128 ? 13 : 14; }
+// complex64: two CTAs of 256 threads keep the 16 amplitudes of a stage in 128
+// registers a thread (512 circuits of 8-18 qubits: 12.3 ms of device time
+// against 14.2 with one CTA of 512)
+int default_threads_batch(int dtype) { return dtype == EV_C64 ? 256 : 512; }
 
 }  // namespace
 
@@ -1073,7 +1101,7 @@ extern "C" int ev_batch_run(const ev_batch_circuit* items, uint64_t count, const
   const int kcap = max_tile_bits(dtype);
   int from_cache = 0;
   if (kbits <= 0 || threads <= 0) {
-    const std::string key = batch_key(items, count, dtype);
+    const std::string key = batch_key(items, count, dtype, kbits, threads, device_name(dev));
     int ck = 0, ct = 0;
     bool cached;
     {
@@ -1098,7 +1126,7 @@ extern "C" int ev_batch_run(const ev_batch_circuit* items, uint64_t count, const
         sample.push_back(b);
       }
       double best = 1e300;
-      int bk = default_tile_bits_batch(dtype), bt = 512;
+      int bk = default_tile_bits_batch(dtype), bt = default_threads_batch(dtype);
       for (int kc = kcap - 2; kc <= kcap; ++kc)
         for (int tc : {256, 512}) {
           if (kbits > 0 && kc != kbits) continue;
@@ -1125,10 +1153,7 @@ extern "C" int ev_batch_run(const ev_batch_circuit* items, uint64_t count, const
     }
   }
   if (kbits <= 0) kbits = default_tile_bits_batch(dtype);
-  // complex64: two CTAs of 256 threads keep the 16 amplitudes of a stage in
-  // 128 registers a thread (512 circuits of 8-18 qubits: 12.3 ms of device
-  // time against 14.2 with one CTA of 512)
-  if (threads <= 0) threads = dtype == EV_C64 ? 256 : 512;
+  if (threads <= 0) threads = default_threads_batch(dtype);
   if (kbits > kcap) kbits = kcap;
   if (kbits < 4) kbits = 4;
   if (threads != 256 && threads != 512)

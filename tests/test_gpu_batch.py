@@ -273,3 +273,23 @@ def test_staged_batch_classical_control(gpu, tile_bits, threads):
         assert r.classical == bits, i
         assert close64(r.amplitudes, want), (i, c.num_qubits())
         assert np.array_equal(r.shots, O.sample_tree(np.ascontiguousarray(r.amplitudes), i, 100)), i
+
+
+def test_tuned_records_of_other_kernels_and_requests_are_not_read(gpu, tmp_path, monkeypatch):
+    """A record without this revision's key (as the first kernels wrote it)
+    leaves the defaults, and a record tuned under a fixed tile or block size
+    serves only calls that fix the same one."""
+    path = tmp_path / "tune.txt"
+    monkeypatch.setenv("EV_AUTOTUNE_CACHE", str(path))
+    circs = tfim_mix(20, 8, 16, seed=6)
+    _, tuned = batch.run_batch(circs, shots=10, autotune=True)
+    key = path.read_text().split()[0]
+    plain = key[key.index("c64:"):]
+    path.write_text(f"{plain} 12 512\n")
+    _, s = batch.run_batch(circs, shots=10)
+    assert not s["from_cache"] and (s["tile_bits"], s["threads"]) == (13, 256)
+    path.write_text(f"{key} 12 512\n")
+    _, s = batch.run_batch(circs, shots=10)
+    assert s["from_cache"] and (s["tile_bits"], s["threads"]) == (12, 512)
+    _, s = batch.run_batch(circs, shots=10, tile_bits=14)
+    assert not s["from_cache"] and (s["tile_bits"], s["threads"]) == (14, 256)
