@@ -276,35 +276,11 @@ static int launch_tile(ev_state* s, const SegStep& st, const TileOp* dops) {
   }
 }
 
-// Tile bits when the caller names none.  A complex128 pass is bound by the
-// FP64 and integer pipes of the SMs that hold a tile, so a register below
-// 2^19 amplitudes is cut into enough tiles to reach them all, at the price of
-// more passes (a few microseconds each); from 2^20 on, tiles of 2^12 fill
-// the GPU and the fewest passes win.  At 2^19 amplitudes the 128 tiles of
-// 2^12 leave SMs without one, and at 2^21 the 512 are 3.4 an SM where some
-// get four; twice as many tiles of 2^11 are shared out better (6.7 of 7 at
-// 2^21): tiles of 2^12 / 2^11, ms, random layers of depth 12, Haar layers of
-// depth 8, QFT: 19 qubits 2.39 / 2.38, 1.25 / 1.18, 0.53 / 0.49; 21 qubits
-// 8.69 / 8.11, 4.65 / 4.15, 1.89 / 1.74; but 20 qubits 4.28 / 4.75, 2.30 /
-// 2.30, 0.91 / 0.93 and 22 qubits 15.4 / 17.6, 8.31 / 8.36, 3.32 / 3.42.
-// The other lines, complex128, ms per depth-20 random-layer circuit (depth 10
-// at 10 qubits), tiles of 2^8 / 2^10 / 2^12: 10 qubits 0.21 / 0.41 / -; 14
-// qubits 0.61 / 1.09 / 2.94; 17 qubits 1.10 / 1.82 / 3.60; 18 qubits 2.24 /
-// 2.00 / 5.5; 19 qubits 4.2 / 4.1 / 4.0; 20 qubits 8.4 / 8.5 / 7.4.
-// complex64 (2^8 / 2^10 / 2^12 / 2^13, the last two in stages): 14 qubits 0.21 /
-// 0.23 / 0.38 / 0.66; 17 qubits 0.36 / 0.32 / 0.47 / 0.82; 18 qubits 0.62 /
-// 0.40 / 0.55 / 0.87; 20 qubits - / 1.30 / 0.85 / 1.08; 22 qubits, depth 10,
-// - / 2.5 / 1.39 / 1.49; 25-qubit QFT - / 12.9 / 3.5 / 3.2.
-int default_tile_bits(int dtype, int n) {
-  if (dtype == EV_C128) return n <= 17 ? 8 : n <= 18 ? 10 : n == 19 || n == 21 ? 11 : 12;
-  return n <= 15 ? 8 : n <= 19 ? 10 : n <= 22 ? 12 : 13;
-}
-
 // Plans a gate run into tile passes; plans and records go into the blob.
 int plan_tiled(ev_state* s, const ev_circuit* c, uint64_t first, uint64_t last, int tile_bits,
                PlanBlob* blob, std::vector<SegStep>* out) {
   const int n = int(s->n);
-  int k = tile_bits > 0 ? tile_bits : default_tile_bits(s->dtype, n);
+  int k = tile_bits > 0 ? tile_bits : default_tile_bits(s->dtype, n, s->num_sms);
   const int kcap = s->dtype == EV_C128 ? 13 : 14;  // tile + records within 227 KiB
   if (k > kcap) k = kcap;
   if (k < 2) k = 2;

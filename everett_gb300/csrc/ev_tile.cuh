@@ -654,6 +654,37 @@ inline std::vector<Pass> plan_passes(const ev_circuit* c, uint64_t first, uint64
   return passes;
 }
 
+// How much longer the fullest SM works than the average one when `tiles` are
+// dealt out over them.
+inline double tile_imbalance(double tiles, int sms) { return std::ceil(tiles / sms) * sms / tiles; }
+
+// Tile bits when the caller names none.  A complex128 pass is bound by the
+// FP64 and integer pipes of the SMs that hold a tile, so a register below
+// 2^19 amplitudes is cut into enough tiles to reach them all, at the price of
+// more passes (a few microseconds each); above, tiles of 2^12 take the fewest
+// passes, and tiles of 2^11 about a tenth more time in all.  So 2^11 is taken
+// where it shares the work out better by more than that, and where 2^12
+// leaves SMs without a tile.  On 152 SMs that is 19 qubits (128 tiles of
+// 2^12) and 21 (512 tiles: 3.4 an SM where some get four, 1024 are 6.7 of
+// seven): tiles of 2^12 / 2^11, ms, random layers of depth 12, Haar layers of
+// depth 8, QFT: 19 qubits 2.39 / 2.38, 1.25 / 1.18, 0.53 / 0.49; 21 qubits
+// 8.69 / 8.11, 4.65 / 4.15, 1.89 / 1.74; but 20 qubits 4.28 / 4.75, 2.30 /
+// 2.30, 0.91 / 0.93 and 22 qubits 15.4 / 17.6, 8.31 / 8.36, 3.32 / 3.42.
+// The other lines, complex128, ms per depth-20 random-layer circuit (depth 10
+// at 10 qubits), tiles of 2^8 / 2^10 / 2^12: 10 qubits 0.21 / 0.41 / -; 14
+// qubits 0.61 / 1.09 / 2.94; 17 qubits 1.10 / 1.82 / 3.60; 18 qubits 2.24 /
+// 2.00 / 5.5; 19 qubits 4.2 / 4.1 / 4.0; 20 qubits 8.4 / 8.5 / 7.4.
+// complex64 (2^8 / 2^10 / 2^12 / 2^13, the last two in stages): 14 qubits 0.21 /
+// 0.23 / 0.38 / 0.66; 17 qubits 0.36 / 0.32 / 0.47 / 0.82; 18 qubits 0.62 /
+// 0.40 / 0.55 / 0.87; 20 qubits - / 1.30 / 0.85 / 1.08; 22 qubits, depth 10,
+// - / 2.5 / 1.39 / 1.49; 25-qubit QFT - / 12.9 / 3.5 / 3.2.
+inline int default_tile_bits(int dtype, int n, int sms) {
+  if (dtype == EV_C64) return n <= 15 ? 8 : n <= 19 ? 10 : n <= 22 ? 12 : 13;
+  if (n <= 18) return n <= 17 ? 8 : 10;
+  const double tiles = std::ldexp(1.0, n - 12);
+  return tiles < sms || tile_imbalance(tiles, sms) > 1.1 * tile_imbalance(2 * tiles, sms) ? 11 : 12;
+}
+
 inline void encode_op(const ev_circuit* c, const ev_op& op, uint64_t tset, const int* local,
                       TileOp* out) {
   std::memset(out, 0, sizeof(*out));

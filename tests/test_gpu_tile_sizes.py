@@ -105,3 +105,11 @@ def test_stages_equal_sweeps(gpu, monkeypatch, n, tile_bits):
     want, _, _ = O.run_seeded(c, 0, parallel=True)
     want = want / np.linalg.norm(want)
     assert np.max(np.abs(staged - want)) < 1e-5
+
+
+@pytest.mark.parametrize("n", [15, 20, 23])
+def test_default_tiles_at_the_other_edges(gpu, n):
+    """The sizes beside the remaining edges: 15 and 20 qubits (complex64
+    tiles of 2^8 | 2^10 and 2^10 | 2^12; complex128 between two registers in
+    tiles of 2^11), 23 (complex64 tiles of 2^13)."""
+    test_default_tiles_bit_exact(gpu, n)

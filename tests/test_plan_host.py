@@ -41,3 +41,26 @@ def test_planning_is_linear_in_the_gates(program):
     assert len(rows) == 12
     for n, idle, reorder, short, long in rows:
         assert float(long) <= 4 * float(short), (n, idle, reorder, short, long)
+
+
+@pytest.mark.parametrize("sms", [76, 132, 148, 152, 160, 304])
+def test_default_tiles_follow_the_sms(program, sms):
+    """complex128 tiles of 2^11 or 2^12 by how evenly this GPU's SMs share
+    them: never 2^12 where it leaves an SM without a tile, 2^11 exactly where
+    the fullest SM's excess shrinks by more than a tenth.  On 152 SMs the
+    sizes measured: 19 and 21 qubits."""
+    r = subprocess.run([str(program), "tiles", str(sms)], capture_output=True, text=True, timeout=60)
+    assert r.returncode == 0, r.stderr
+    bits = {int(n): (int(a), int(b)) for n, a, b in (line.split() for line in r.stdout.splitlines())}
+
+    def excess(tiles):
+        return -(-tiles // sms) * sms / tiles
+
+    for n in range(19, 35):
+        tiles = 1 << (n - 12)
+        small = tiles < sms or excess(tiles) > 1.1 * excess(2 * tiles)
+        assert bits[n][0] == (11 if small else 12), n
+    if sms == 152:
+        want = [8] * 17 + [10, 11, 12, 11] + [12] * 13
+        assert [bits[n][0] for n in range(1, 35)] == want
+    assert [bits[n][1] for n in range(1, 35)] == [8] * 15 + [10] * 4 + [12] * 3 + [13] * 12
