@@ -407,7 +407,7 @@ __global__ void __launch_bounds__(NT, STAGES ? 512 / NT : NT == 256 ? 3 : 2) k_b
       while (j < cnt) {
         const BatchOp* rec = srec + j;
         const BatchOp op = *rec;
-        // chains (run > 1) are formed only in circuits without classical ops
+        // a record that a prefix gates has a run of 1 (plan_circuit)
         const uint32_t run = op.run > 1 ? op.run : 1;
         if (j + run > cnt) break;  // the next window starts at this chain
         j += run;
@@ -682,23 +682,32 @@ void plan_circuit(const ev_circuit* c, int kmax, bool c64, uint32_t window, Circ
       }
     out->plans.push_back(plan);
     out->passes.push_back({uint32_t(out->ops.size()), uint32_t(p.ops.size())});
-    // the pass's gate records, chained as the tile pass chains them (not in
-    // circuits with measurements or classical control, whose records run one
-    // by one in the classical register's order)
+    // the pass's gate records, in stages or chained as the tile pass chains
+    // them.  In circuits with measurements or classical control a stage ends
+    // at a measurement or an IfClassic prefix, and the record that a prefix
+    // gates is a stage of its own; chains are not formed there.
     recs.assign(p.ops.size(), TileOp{});
+    size_t from = 0;  // first record not in a stage
+    auto stage_to = [&](size_t to) {
+      if (stages && to > from) mark_stages(&recs[from], to - from, k, window);
+      from = to;
+    };
+    bool gated = false;
     for (size_t j = 0; j < p.ops.size(); ++j) {
       const ev_op& src = c->ops[p.ops[j]];
-      if (src.kind == EV_OP_MEASURE || src.kind == EV_OP_IF) continue;
-      encode_op(c, src, p.tset, local, &recs[j]);
-      if (c64) pack_f32_matrix(recs[j].m, recs[j].kind == T_1Q ? 8 : 32);
-      if (stages && out->classical) mark_stages(&recs[j], 1, k, 1);
+      const bool gate = src.kind != EV_OP_MEASURE && src.kind != EV_OP_IF;
+      if (!gate || gated) stage_to(j);
+      if (gate) {
+        encode_op(c, src, p.tset, local, &recs[j]);
+        if (c64) pack_f32_matrix(recs[j].m, recs[j].kind == T_1Q ? 8 : 32);
+        if (gated) stage_to(j + 1);
+      } else {
+        from = j + 1;
+      }
+      gated = src.kind == EV_OP_IF;
     }
-    if (!out->classical) {
-      if (stages)
-        mark_stages(recs.data(), recs.size(), k, window);
-      else
-        mark_chains(recs.data(), recs.size(), chains, window);
-    }
+    stage_to(p.ops.size());
+    if (!stages && !out->classical) mark_chains(recs.data(), recs.size(), chains, window);
     for (size_t jj = 0; jj < p.ops.size(); ++jj) {
       const ev_op& src = c->ops[p.ops[jj]];
       if (src.kind == EV_OP_MEASURE || src.kind == EV_OP_IF) {

@@ -293,3 +293,20 @@ def test_tuned_records_of_other_kernels_and_requests_are_not_read(gpu, tmp_path,
     assert s["from_cache"] and (s["tile_bits"], s["threads"]) == (12, 512)
     _, s = batch.run_batch(circs, shots=10, tile_bits=14)
     assert not s["from_cache"] and (s["tile_bits"], s["threads"]) == (14, 256)
+
+
+@pytest.mark.parametrize("n", [11, 13])
+def test_a_measurement_does_not_split_its_circuit(gpu, n):
+    """complex64 circuits with a measurement run their gates in the stages
+    that the same gates without one take: a stage ends at the measurement
+    only, not at every record (which took twice the device time)."""
+    def device_ms(circs):
+        return min(batch.run_batch(circs, shots=16, dtype="complex64", tile_bits=13,
+                                   threads=256)[1]["device_ms"] for _ in range(5))
+    plain, measured = [], []
+    for seed in range(32):
+        body = workloads.random_layers(n, 12, seed)
+        plain.append(body)
+        c = Circuit.with_classical(n, 1)
+        measured.append(c.compose(body).measure(0, 0))
+    assert device_ms(measured) <= 1.3 * device_ms(plain)
