@@ -792,20 +792,21 @@ extern "C" int ev_normalize(ev_state* s) {
 // t of norm_sqr(a[t * 2^m + c]), each sum taken in increasing t from 0.0 --
 // the order of the basis loop in phase_estimation.rs:97-110
 // (most_probable_phase).  One thread per c; the loads of a warp are
-// consecutive amplitudes, kMarginalLoads of them in flight.
+// consecutive amplitudes.  128 bytes of them are on their way while as many
+// are summed: with few sums (2^m threads) a thread's chain of loads and adds
+// is all there is, and loading, then summing each group took twice as long
+// (complex128, 24 qubits, m = 8: 30.7 ms, now 13.8).
 //
-// complex64 is bound by the FP64 pipe, which also runs the f32 -> f64
-// conversions: 5 instructions per amplitude with the squares formed there.
-// The square of a float fits 48 bits, so it is formed exactly on the integer
-// pipes (square_f64) and the same two sums remain: same bits, 28 qubits, m =
-// 20: 2.46 -> 1.03 ms.
-constexpr int kMarginalLoads = 8;
+// complex64 with many sums is bound by the FP64 pipe, which also runs the f32
+// -> f64 conversions: 5 instructions per amplitude with the squares formed
+// there.  The square of a float fits 48 bits, so it is formed exactly on the
+// integer pipes (square_f64) and the same two sums remain: same bits, 28
+// qubits, m = 20, a call: 2.53 -> 1.13 ms.
 
 // x * x as an f64 (exact).
 __device__ __forceinline__ double square_f64(float x) {
   const uint32_t u = __float_as_uint(x) & 0x7FFFFFFFu;
-  if (u - 0x00800000u >= 0x7F000000u) {  // zero, subnormal, infinite, NaN
-    if (u == 0u) return 0.0;
+  if (u - 0x00800000u >= 0x7F000000u && u != 0u) {  // subnormal, infinite, NaN
     const double d = double(x);
     return __dmul_rn(d, d);
   }
@@ -813,9 +814,11 @@ __device__ __forceinline__ double square_f64(float x) {
   const uint64_t p = m * m;  // in [2^46, 2^48)
   const uint32_t top = uint32_t(p >> 47);
   // the significand's leading one, at bit 52 after the shift, completes the
-  // exponent field
-  return __longlong_as_double(
-      (long long)((uint64_t(2u * (u >> 23) + 768u + top) << 52) + (p << (6u - top))));
+  // exponent field.  A zero is selected, not branched to, in the high word (p
+  // << 6 leaves its low word zero): states with many zeros took 2.79 ms at 28
+  // qubits with a branch, dense ones 1.10.
+  const uint64_t bits = (uint64_t(2u * (u >> 23) + 768u + top) << 52) + (p << (6u - top));
+  return __hiloint2double(u == 0u ? 0 : int(bits >> 32), int(uint32_t(bits)));
 }
 __device__ __forceinline__ double marginal_term(float2 a) {
   return __dadd_rn(square_f64(a.x), square_f64(a.y));  // as nsq: both products are exact
@@ -827,16 +830,29 @@ __global__ void __launch_bounds__(256)
     k_marginal_low(const V* __restrict__ s, uint32_t m, uint64_t iters, double* __restrict__ out) {
   const uint64_t c = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x;
   if (c >= (uint64_t(1) << m)) return;
+  constexpr int LOADS = 128 / sizeof(V);
+  const V* p = s + c;
   double acc = 0.0;
-  for (uint64_t t0 = 0; t0 < iters; t0 += kMarginalLoads) {
-    V v[kMarginalLoads];
-#pragma unroll
-    for (int j = 0; j < kMarginalLoads; ++j)
-      if (t0 + j < iters) v[j] = s[((t0 + j) << m) | c];
-#pragma unroll
-    for (int j = 0; j < kMarginalLoads; ++j)
-      if (t0 + j < iters) acc = __dadd_rn(acc, marginal_term(v[j]));
+  if (iters < LOADS) {
+    for (uint64_t t = 0; t < iters; ++t) acc = __dadd_rn(acc, marginal_term(p[t << m]));
+    out[c] = acc;
+    return;
   }
+  V v[LOADS];
+#pragma unroll
+  for (int j = 0; j < LOADS; ++j) v[j] = p[uint64_t(j) << m];
+#pragma unroll 2
+  for (uint64_t t = LOADS; t < iters; t += LOADS) {  // iters is a power of two
+    V w[LOADS];
+#pragma unroll
+    for (int j = 0; j < LOADS; ++j) w[j] = p[(t + uint64_t(j)) << m];
+#pragma unroll
+    for (int j = 0; j < LOADS; ++j) acc = __dadd_rn(acc, marginal_term(v[j]));
+#pragma unroll
+    for (int j = 0; j < LOADS; ++j) v[j] = w[j];
+  }
+#pragma unroll
+  for (int j = 0; j < LOADS; ++j) acc = __dadd_rn(acc, marginal_term(v[j]));
   out[c] = acc;
 }
 

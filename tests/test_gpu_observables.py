@@ -285,3 +285,50 @@ def test_more_terms_than_results_wait_on_the_device(gpu, dtype):
         xm, zm = p.masks()
         want = O.pauli_expectation(ref, xm, zm, p.neg)
         assert abs(g - want) < 1e-12, (dtype, str(p), g, want)
+
+
+@pytest.mark.parametrize("dtype", ["complex128", "complex64"])
+def test_marginal_sums_of_every_length(gpu, dtype):
+    """Sums shorter than, equal to and longer than the amplitudes that are on
+    their way together, over zeros and dense values: the f64 sum in basis
+    order (complex128 squares as the oracle's norm_sqr: x x + y y, the second
+    product rounded into the first's sum once or twice)."""
+    n = 12
+    rng = np.random.default_rng(5)
+    for zeros in (0.0, 0.6, 0.99):
+        amps = rng.normal(size=1 << n) + 1j * rng.normal(size=1 << n)
+        amps[rng.uniform(size=1 << n) < zeros] = 0.0
+        if dtype == "complex64":
+            amps = amps.astype(np.complex64).astype(np.complex128)
+        st = State.from_amplitudes(amps, dtype=dtype)
+        terms = amps.real ** 2 + amps.imag ** 2
+        for m in range(n + 1):
+            want = np.zeros(1 << m)
+            for row in terms.reshape(-1, 1 << m):
+                want = want + row
+            got = st.marginal_low(m)
+            if dtype == "complex64":  # exact squares
+                assert np.array_equal(got, want), (zeros, m)
+            else:  # one rounding more or less per term
+                assert np.max(np.abs(got - want)) <= 2.0 ** -51 * (1 << (n - m)) * terms.max(), (zeros, m)
+
+
+def test_marginal_times_by_length_and_content(gpu):
+    """Few long sums: four times the terms take at most five times as long
+    (the loads of a register beyond the L2 cache stay ahead of the adds), and
+    a state of zeros takes as long as a dense one."""
+    import time
+
+    def seconds(st, m):
+        best = 1e9
+        for _ in range(5):
+            t = time.perf_counter()
+            st.marginal_low(m)
+            best = min(best, time.perf_counter() - t)
+        return best
+
+    short, long = State.zero(22, "complex128"), State.zero(24, "complex128")
+    assert seconds(long, 8) <= 5.0 * seconds(short, 8)
+    sparse = State.zero(24, "complex64")
+    dense = CudaStateVectorBackend.run(workloads.random_layers(24, 1, seed=2), dtype="complex64").state()
+    assert seconds(sparse, 12) <= 1.2 * seconds(dense, 12)
