@@ -22,6 +22,8 @@
 
 #include <type_traits>
 
+#include <cmath>
+
 #include "ev_device.cuh"
 #include "ev_internal.h"
 #include "ev_softpair.cuh"
@@ -31,6 +33,8 @@ namespace ev {
 template <typename V>
 struct M1 {
   V m0, m1, m2, m3;
+  uint32_t finite;         // complex128: no entry is infinite or NaN
+  uint32_t one_magnitude;  // complex128: the four real parts share one (H)
 };
 template <typename V>
 struct M2 {
@@ -45,13 +49,17 @@ template <typename V>
 M1<V> to_m1(const double m[8]);
 template <>
 M1<double2> to_m1<double2>(const double m[8]) {
+  uint32_t finite = 1;
+  for (int e = 0; e < 8; ++e) finite &= finite_bits(m[e]);
+  uint32_t one = 1;
+  for (int e = 2; e < 8; e += 2) one &= uint32_t(std::fabs(m[e]) == std::fabs(m[0]));
   return {make_double2(m[0], m[1]), make_double2(m[2], m[3]), make_double2(m[4], m[5]),
-          make_double2(m[6], m[7])};
+          make_double2(m[6], m[7]), finite, one};
 }
 template <>
 M1<float2> to_m1<float2>(const double m[8]) {
   return {make_float2(float(m[0]), float(m[1])), make_float2(float(m[2]), float(m[3])),
-          make_float2(float(m[4]), float(m[5])), make_float2(float(m[6]), float(m[7]))};
+          make_float2(float(m[4]), float(m[5])), make_float2(float(m[6]), float(m[7])), 1u, 0u};
 }
 
 __device__ __forceinline__ bool skip(const uint8_t* pred) { return pred != nullptr && *pred == 0; }
@@ -99,9 +107,11 @@ __device__ __forceinline__ void pair_update_soft(double2* __restrict__ s, uint64
     // a sparse state (every one is until its last qubit has been rotated):
     // nothing to compute or to write.  Zeros are outside the integer-pipe
     // domain and took the FP64 pipe: dense gates at 26 qubits while half the
-    // register is still in |0>, 1298 us a gate, 190 now.
-    if (zero_amp(a0) && zero_amp(a1)) return;
-    soft_pair<KIND>(a0, a1, f, true);
+    // register is still in |0>, 1298 us a gate, 190 now.  Real matrices, whose
+    // products cost less, ask once an operand is out of the domain (22 qubits,
+    // no zeros: 25.6 us a gate, 26.6 asked first).
+    if (KIND != K1_REAL && zero_amp(a0) && zero_amp(a1)) return;
+    if (!soft_pair<KIND>(a0, a1, f, true)) return;
     s[i0] = a0;
     s[i1] = a1;
   }
@@ -109,11 +119,6 @@ __device__ __forceinline__ void pair_update_soft(double2* __restrict__ s, uint64
 
 // A real matrix whose entries share one magnitude (H): m2 a0 and m3 a1 are
 // m0 a0 and m1 a1 up to sign, so 4 products on the integer pipes serve the 8.
-__device__ __forceinline__ bool one_magnitude(const SoftM1& f) {
-  const uint64_t m = softfp::to_bits(f.m0.x) << 1;
-  return (softfp::to_bits(f.m1.x) << 1) == m && (softfp::to_bits(f.m2.x) << 1) == m &&
-         (softfp::to_bits(f.m3.x) << 1) == m;
-}
 __device__ __forceinline__ void pair_update_hadamard(double2* __restrict__ s, uint64_t i0,
                                                      uint64_t i1, const SoftM1& f, uint64_t flip0,
                                                      uint64_t flip1) {
@@ -168,9 +173,9 @@ __global__ void __launch_bounds__(256) k_pair(V* __restrict__ s, uint64_t npairs
         return;
       }
     }
-    const SoftM1 f = soft_matrix<KIND>(m.m0, m.m1, m.m2, m.m3);
+    const SoftM1 f = soft_matrix<KIND>(m.m0, m.m1, m.m2, m.m3, m.finite);
     if constexpr (KIND == K1_REAL) {
-      if (f.ok && one_magnitude(f)) {
+      if (f.ok & m.one_magnitude) {
         const uint64_t sign = uint64_t(1) << 63;
         const uint64_t flip0 = (softfp::to_bits(f.m0.x) ^ softfp::to_bits(f.m2.x)) & sign;
         const uint64_t flip1 = (softfp::to_bits(f.m1.x) ^ softfp::to_bits(f.m3.x)) & sign;
@@ -224,7 +229,7 @@ __global__ void __launch_bounds__(256) k_pair_shfl(V* __restrict__ s, uint64_t l
   // the lane's matrix row: (m0, m1) for new0, (m2, m3) for new1
   const V r0 = hi ? m.m2 : m.m0, r1 = hi ? m.m3 : m.m1;
   if constexpr (std::is_same<V, double2>::value && (KIND == K1_DENSE || KIND == K1_REAL)) {
-    const SoftM1 f = soft_matrix<KIND>(m.m0, m.m1, m.m2, m.m3);
+    const SoftM1 f = soft_matrix<KIND>(m.m0, m.m1, m.m2, m.m3, m.finite);
     if (f.ok) {  // uniform: the row's factors on the integer pipes
       const softfp::Unpacked u0 = hi ? f.u2 : f.u0, u1 = hi ? f.u3 : f.u1;
       for (uint64_t j = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; j < len; j += stride) {
@@ -274,13 +279,13 @@ __global__ void __launch_bounds__(256) k_pair_shfl(V* __restrict__ s, uint64_t l
 // Coalesced for every k; same products as the pair form.
 template <typename V>
 __global__ void __launch_bounds__(256) k_diag(V* __restrict__ s, uint64_t len, int k, V d0, V d1,
-                                              const uint8_t* pred) {
+                                              uint32_t finite, const uint8_t* pred) {
   if (skip(pred)) return;
   const uint64_t stride = uint64_t(gridDim.x) * blockDim.x;
   if constexpr (std::is_same<V, double2>::value) {
     const softfp::Unpacked u0 = softfp::unpack(d0.y), u1 = softfp::unpack(d1.y);
     // products on the integer pipes, as ev_softpair.cuh
-    if (u0.ok & u1.ok & finite_bits(d0.x) & finite_bits(d1.x)) {
+    if (finite & u0.ok & u1.ok) {
       for (uint64_t j = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; j < len; j += stride) {
         const bool one = (j >> k) & 1;
         s[j] = soft_diag(one ? d1 : d0, one ? u1 : u0, s[j]);
@@ -317,7 +322,7 @@ __global__ void __launch_bounds__(256) k_ctrl(V* __restrict__ s, uint64_t count,
         return;
       }
     }
-    const SoftM1 f = soft_matrix<KIND>(m.m0, m.m1, m.m2, m.m3);
+    const SoftM1 f = soft_matrix<KIND>(m.m0, m.m1, m.m2, m.m3, m.finite);
     if (f.ok) {
       for (uint64_t i = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < count; i += stride) {
         uint64_t j = i;
@@ -517,7 +522,8 @@ static void go_apply1(ev_state* s, Kind1 kind, uint64_t k, const double m[8], co
     case K1_ANTI: k_pair<K1_ANTI><<<g, 256, 0, s->stream>>>(a, npairs, int(k), mm, pred); break;
     case K1_PHASE: k_pair<K1_PHASE><<<g, 256, 0, s->stream>>>(a, npairs, int(k), mm, pred); break;
     case K1_DIAG:
-      k_diag<<<grid_for(s, s->len()), 256, 0, s->stream>>>(a, s->len(), int(k), mm.m0, mm.m3, pred);
+      k_diag<<<grid_for(s, s->len()), 256, 0, s->stream>>>(a, s->len(), int(k), mm.m0, mm.m3, mm.finite,
+                                                           pred);
       break;
     case K1_IDENT: break;
   }

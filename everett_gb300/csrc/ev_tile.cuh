@@ -115,7 +115,7 @@ template <int K1, typename Op>
 __device__ __forceinline__ void tile_1q_soft(double2* t, uint32_t count, const Op& op,
                                              const double* mm) {
   const SoftM1 f = soft_matrix<K1>(ldm<double2>(mm, 0), ldm<double2>(mm, 1), ldm<double2>(mm, 2),
-                                   ldm<double2>(mm, 3));
+                                   ldm<double2>(mm, 3), rec_sok(op));
   if (!f.ok) {  // uniform across the block
     tile_1q_fp64<K1>(t, count, op, mm);
     return;
