@@ -185,9 +185,6 @@ struct PauliChannel {
   uint8_t second[EV_MAX_KRAUS], swap[EV_MAX_KRAUS], neg[EV_MAX_KRAUS];
 };
 
-__device__ __forceinline__ bool is_zero(double2 x) {  // tested as bits, off the FP64 pipe
-  return ((softfp::to_bits(x.x) | softfp::to_bits(x.y)) << 1) == 0;
-}
 // RN(c RN(c x)); a zero stays itself, an operand outside the integer-pipe
 // domain takes the FP64 pipe
 __device__ __forceinline__ double twice(double c, const softfp::Unpacked& cu, double x) {
@@ -283,7 +280,7 @@ __global__ void __launch_bounds__(kDmThreads, 3)
     double2 e[4] = {rho[r0 * dim + c0], rho[r0 * dim + c1], rho[r1 * dim + c0], rho[r1 * dim + c1]};
     // a block of zeros stays one under a finite matrix (most of rho until
     // every qubit has been rotated; a zero operand would take the FP64 pipe)
-    if ((!GATE || skip_zeros) && (is_zero(e[0]) & is_zero(e[1]) & is_zero(e[2]) & is_zero(e[3])))
+    if ((!GATE || skip_zeros) && (zero_amp(e[0]) & zero_amp(e[1]) & zero_amp(e[2]) & zero_amp(e[3])))
       continue;
     if (GATE) {
       if ((r0 & mask) == mask) {
