@@ -20,22 +20,24 @@
 
 namespace ev {
 
-// Re and Im of (mr + i mi) (xr + i xi)
+// Re and Im of (mr + i mi) (xr + i xi).  Both are x's real part times the one
+// part of m plus its imaginary part times (-mi, mr): two lanes of one form.
 inline double product_re(double mr, double mi, double xr, double xi) {
-  return std::fma(mr, xr, -(mi * xi));
+  return std::fma(mr, xr, -mi * xi);
 }
 inline double product_im(double mr, double mi, double xr, double xi) {
   return std::fma(mi, xr, mr * xi);
 }
 
 // (x, y) <- (m0 x + m1 y, m2 x + m3 y) over two rows of n complex values
-inline void mix_rows(const double* m, double* x, double* y, int n) {
+inline void mix_rows(const double* m, double* __restrict__ x, double* __restrict__ y, int n) {
+  const double a = m[0], ai = m[1], b = m[2], bi = m[3], c = m[4], ci = m[5], d = m[6], di = m[7];
   for (int i = 0; i < 2 * n; i += 2) {
     const double xr = x[i], xi = x[i + 1], yr = y[i], yi = y[i + 1];
-    x[i] = product_re(m[0], m[1], xr, xi) + product_re(m[2], m[3], yr, yi);
-    x[i + 1] = product_im(m[0], m[1], xr, xi) + product_im(m[2], m[3], yr, yi);
-    y[i] = product_re(m[4], m[5], xr, xi) + product_re(m[6], m[7], yr, yi);
-    y[i + 1] = product_im(m[4], m[5], xr, xi) + product_im(m[6], m[7], yr, yi);
+    x[i] = product_re(a, ai, xr, xi) + product_re(b, bi, yr, yi);
+    x[i + 1] = product_im(a, ai, xr, xi) + product_im(b, bi, yr, yi);
+    y[i] = product_re(c, ci, xr, xi) + product_re(d, di, yr, yi);
+    y[i + 1] = product_im(c, ci, xr, xi) + product_im(d, di, yr, yi);
   }
 }
 
