@@ -365,8 +365,9 @@ struct TcShape {
   // k_fused_tc: TF32 keeps the high parts of A in TMEM, in the K columns
   // above the accumulator.  They are read by two of the three products, and
   // without them a CTA takes 65 KiB of shared memory instead of 97: three
-  // CTAs per SM instead of two (28 qubits: 996 us a pass, 816 now,
-  // 642 at the copy bandwidth).
+  // CTAs per SM instead of two (28 qubits: 996 -> 816 us a pass, 708 with
+  // the low-qubit accesses and operands written as shared memory; 642 at the
+  // copy bandwidth).
   static constexpr bool kHiInTmem = VAR == EV_FUSED_TF32X3;
   static constexpr int TC_SMEM = SMEM - (kHiInTmem ? A_BYTES : 0);
   static constexpr int TC_TMEM_COLS = kHiInTmem ? 2 * K : TMEM_COLS;
