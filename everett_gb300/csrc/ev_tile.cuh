@@ -604,10 +604,12 @@ inline bool moves_only(const ev_op& op) {
 // qubits.
 //
 // Pending ops form a linked list: a pass unlinks what joins and walks over
-// what it leaves, at most kPlanWindow ops, so planning is linear in the ops
-// (10 qubits, k = 8, 400 000 gates: 24 ms; with what is left copied once per
-// pass 11.3 s).
-constexpr int kPlanWindow = 4096;
+// what it leaves until every qubit in use is blocked (10 qubits, k = 8, 400
+// 000 gates: 24 ms; with what is left copied once per pass 11.3 s).  In
+// circuit order it leaves at most kPlanWindow ops, which keeps planning
+// linear whatever the circuit and changes no bit; a reordered plan's
+// roundings depend on its passes, so there the walk isn't cut.
+constexpr size_t kPlanWindow = 4096;
 
 inline std::vector<Pass> plan_passes(const ev_circuit* c, uint64_t first, uint64_t last, int n,
                                      int k, int L, uint64_t max_ops = 48, bool reorder = false) {
@@ -632,9 +634,10 @@ inline std::vector<Pass> plan_passes(const ev_circuit* c, uint64_t first, uint64
     Pass p;
     uint64_t set = low, blocked = 0;
     bool behind = false;  // an arithmetic op has been left behind
-    int left = 0;         // ops left behind
+    size_t left = 0;      // ops left behind
     size_t* link = &head;
-    while (*link != end && p.ops.size() < max_ops && blocked != everything && left < kPlanWindow) {
+    while (*link != end && p.ops.size() < max_ops && blocked != everything &&
+           (reorder || left < kPlanWindow)) {
       Pending& e = pending[*link];
       if ((e.all & blocked) == 0 && (e.moves || !behind) && popc(set | e.data) <= k) {
         set |= e.data;

@@ -88,7 +88,7 @@ std::vector<Pass> rule(const ev_circuit* c, int n, int k, int L, uint64_t max_op
       for (uint32_t i = 0; o.kind == EV_OP_CONTROLLED && i < o.nctrl; ++i)
         all |= uint64_t(1) << c->ctrl_pool[o.ctrl_off + i];
       const bool may_jump = reorder || moves[j] || !behind;
-      if (rest.size() < size_t(kPlanWindow) && p.ops.size() < max_ops && !(all & blocked) &&
+      if ((reorder || rest.size() < kPlanWindow) && p.ops.size() < max_ops && !(all & blocked) &&
           may_jump && __builtin_popcountll(set | data) <= k) {
         set |= data;
         p.ops.push_back(j);
@@ -163,7 +163,7 @@ int same() {
   // that could
   for (bool reorder : {false, true}) {
     Builder b;
-    for (int i = 0; i < kPlanWindow + 300; ++i) b.two(i & 1 ? 0 : 2, 8, 9 + (i & 3));
+    for (size_t i = 0; i < kPlanWindow + 300; ++i) b.two(i & 1 ? 0 : 2, 8, 9 + (i & 3));
     for (int q = 0; q < 6; ++q) b.two(0, q, q + 1);
     check(b, 13, 4, 2, 48, reorder);
     Builder w = layers(13, 2 * kPlanWindow, -1);  // one pass whatever its length
